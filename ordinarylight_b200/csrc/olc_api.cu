@@ -859,15 +859,16 @@ void write_scene_records(olc_context* ctx, const olc_scene_desc* d, ResidentScen
       const uint32_t m = d->instance_mesh[i];
       const uint32_t v0 = d->mesh_vertex_offset[m];
       for (uint32_t lt = 0; lt < mesh_triangles(d, m); ++lt, ++t) {
+        float3 corner[3];
         for (int c = 0; c < 3; ++c) {
           uint32_t vi = v0 + d->indices[3ull * (d->mesh_triangle_offset[m] + lt) + c];
-          float3 p = xform_point(mo, make_float3(d->vertices[3ull * vi], d->vertices[3ull * vi + 1],
-                                                 d->vertices[3ull * vi + 2]));
+          corner[c] = xform_point(mo, make_float3(d->vertices[3ull * vi], d->vertices[3ull * vi + 1],
+                                                  d->vertices[3ull * vi + 2]));
           float3 nn = normalize(xform_normal_by_inverse(
               mw, make_float3(d->normals[3ull * vi], d->normals[3ull * vi + 1], d->normals[3ull * vi + 2])));
-          fv[3 * t + c] = make_float4(p.x, p.y, p.z, 0.0f);
           fn[3 * t + c] = make_float4(nn.x, nn.y, nn.z, 0.0f);
         }
+        set_triangle(fv.data() + 3 * t, corner[0], corner[1], corner[2]);
         fpacked[t] = r.prim_offset + lt;
         fowner[t] = inst0 + L.local_of[i];
       }

@@ -359,11 +359,13 @@ __global__ void k_reorder_triangles(const uint32_t* __restrict__ order, uint32_t
   if (s >= nt) return;
   uint32_t t = order[s];
   uint32_t dst = slot_base + s;
+  float3 v[3];
   for (int k = 0; k < 3; ++k) {
     uint32_t vi = indices[3 * t + k];
-    tri_verts[3ull * dst + k] = make_float4(vertices[3 * vi + 0], vertices[3 * vi + 1], vertices[3 * vi + 2], 0.0f);
+    v[k] = f3(vertices[3 * vi + 0], vertices[3 * vi + 1], vertices[3 * vi + 2]);
     tri_normals[3ull * dst + k] = make_float4(normals[3 * vi + 0], normals[3 * vi + 1], normals[3 * vi + 2], 0.0f);
   }
+  set_triangle(tri_verts + 3ull * dst, v[0], v[1], v[2]);
   tri_index[dst] = t;
 }
 
@@ -372,7 +374,8 @@ __global__ void k_flat_triangle_boxes(const float4* __restrict__ verts, uint32_t
                                       float4* centers) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float3 a = f3(verts[3ull * i]), b = f3(verts[3ull * i + 1]), c = f3(verts[3ull * i + 2]);
+  float3 a, b, c;
+  load_triangle(verts + 3ull * i, a, b, c);
   float3 l = fminf3(fminf3(a, b), c), h = fmaxf3(fmaxf3(a, b), c);
   lo[i] = make_float4(l.x, l.y, l.z, 0.0f);
   hi[i] = make_float4(h.x, h.y, h.z, 0.0f);
@@ -405,10 +408,14 @@ __global__ void __launch_bounds__(256) k_instance_box_parts(const float* __restr
   const uint2 range = slot_ranges[i];
   uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
   const uint64_t stride = (uint64_t)gridDim.y * blockDim.x;
-  for (uint64_t v = 3ull * range.x + (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; v < 3ull * range.y; v += stride) {
-    const float3 w = xform_point(m, f3(tri_verts[v]));
-    const uint32_t o[3] = {f2ord(w.x), f2ord(w.y), f2ord(w.z)};
-    for (int k = 0; k < 3; ++k) { mn[k] = min(mn[k], o[k]); mx[k] = max(mx[k], o[k]); }
+  for (uint64_t t = range.x + (uint64_t)blockIdx.y * blockDim.x + threadIdx.x; t < range.y; t += stride) {
+    float3 corner[3];
+    load_triangle(tri_verts + 3ull * t, corner[0], corner[1], corner[2]);
+    for (int v = 0; v < 3; ++v) {
+      const float3 w = xform_point(m, corner[v]);
+      const uint32_t o[3] = {f2ord(w.x), f2ord(w.y), f2ord(w.z)};
+      for (int k = 0; k < 3; ++k) { mn[k] = min(mn[k], o[k]); mx[k] = max(mx[k], o[k]); }
+    }
   }
   for (int k = 0; k < 3; ++k) {
     for (int off = 16; off > 0; off >>= 1) {
@@ -698,11 +705,13 @@ __global__ void k_refresh_slots(const float* __restrict__ vertices, const float*
   if (s >= nt) return;
   const uint32_t dst = slot_base + s;
   const uint32_t t = tri_index[dst];
+  float3 v[3];
   for (int k = 0; k < 3; ++k) {
     uint32_t vi = indices[3 * t + k];
-    tri_verts[3ull * dst + k] = make_float4(vertices[3 * vi + 0], vertices[3 * vi + 1], vertices[3 * vi + 2], 0.0f);
+    v[k] = f3(vertices[3 * vi + 0], vertices[3 * vi + 1], vertices[3 * vi + 2]);
     tri_normals[3ull * dst + k] = make_float4(normals[3 * vi + 0], normals[3 * vi + 1], normals[3 * vi + 2], 0.0f);
   }
+  set_triangle(tri_verts + 3ull * dst, v[0], v[1], v[2]);
 }
 
 __global__ void k_refit_init(uint32_t count, int* parent, uint32_t* done) {
@@ -734,12 +743,14 @@ OLC_D void slot_range_box(const float4* tri_verts, int ref, float3& lo, float3& 
   hi = make_float3(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
   if (ref == OLC_EMPTY_CHILD) return;
   const uint32_t first = olc_leaf_first(ref), n = olc_leaf_count(ref);
-  for (uint32_t k = 0; k < n; ++k)
+  for (uint32_t k = 0; k < n; ++k) {
+    float3 p[3];
+    load_triangle(tri_verts + 3ull * (first + k), p[0], p[1], p[2]);
     for (int v = 0; v < 3; ++v) {
-      const float3 p = f3(tri_verts[3ull * (first + k) + v]);
-      lo = fminf3(lo, p);
-      hi = fmaxf3(hi, p);
+      lo = fminf3(lo, p[v]);
+      hi = fmaxf3(hi, p[v]);
     }
+  }
 }
 
 // Union of a node's two child boxes (its own box).

@@ -250,6 +250,21 @@ struct __align__(16) RefVolume {
 };
 static_assert(sizeof(RefVolume) == 288, "RefVolume must match the 72-float scene-description record");
 
+// A triangle slot's vertices: three float4, one per axis, each holding that
+// coordinate of the three vertices (w unused), so that traversal reads the
+// axes in its ray's shear order.
+OLC_HD void load_triangle(const float4* tv, float3& a, float3& b, float3& c) {
+  const float4 x = tv[0], y = tv[1], z = tv[2];
+  a = f3(x.x, y.x, z.x);
+  b = f3(x.y, y.y, z.y);
+  c = f3(x.z, y.z, z.z);
+}
+OLC_HD void set_triangle(float4* tv, float3 a, float3 b, float3 c) {
+  tv[0] = make_float4(a.x, b.x, c.x, 0.0f);
+  tv[1] = make_float4(a.y, b.y, c.y, 0.0f);
+  tv[2] = make_float4(a.z, b.z, c.z, 0.0f);
+}
+
 // One resident scene of the pool: its TLAS root and its lighting.  Emitter
 // indices of the alias table are scene-local (add emitter_base).
 struct __align__(16) SceneRec {
@@ -295,7 +310,7 @@ struct __align__(16) SceneRec {
 struct SceneView {
   const BvhNode* nodes;          // BLAS and TLAS nodes
   const BvhNode4* wide;          // their BVH4 form, same indices (traversal reads only these)
-  const float4* tri_verts;       // 3 float4 per triangle slot (object space)
+  const float4* tri_verts;       // 3 float4 per triangle slot (object space): per axis, that coordinate of the vertices
   const float4* tri_normals;     // 3 float4 per triangle slot (object space)
   const uint32_t* tri_index;     // slot -> mesh-local triangle index (packed index for baked triangles)
   const uint32_t* tri_owner;     // slot -> original instance (baked triangles only)

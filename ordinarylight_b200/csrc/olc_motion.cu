@@ -39,14 +39,14 @@ __global__ void k_world_triangles(SceneView s, const MotionSegment* __restrict__
     const float4* tv = s.tri_verts + 3ull * slot;
     uint32_t packed;
     float3 v[3];
+    load_triangle(tv, v[0], v[1], v[2]);
     if (sg.prim_offset == 0xffffffffu) {
       packed = s.tri_index[slot];
-      for (int k = 0; k < 3; ++k) v[k] = f3(tv[k]);
     } else {
       packed = sg.prim_offset + s.tri_index[slot];
       const InstanceRec& ir = s.instances[sg.instance];
       const Affine o2w{ir.o2w0, ir.o2w1, ir.o2w2};
-      for (int k = 0; k < 3; ++k) v[k] = xform_point(o2w, f3(tv[k]));
+      for (int k = 0; k < 3; ++k) v[k] = xform_point(o2w, v[k]);
     }
     if (packed >= num_packed) continue;
     for (int k = 0; k < 3; ++k) out[3ull * packed + k] = make_float4(v[k].x, v[k].y, v[k].z, 0.0f);

@@ -228,7 +228,11 @@ OLC_D PrimaryVertex primary_vertex(const SceneView& s, const RayQueue& q, const 
   Affine o2w{ir.o2w0, ir.o2w1, ir.o2w2};
   Affine w2o{ir.w2o0, ir.w2o1, ir.w2o2};
   const float4* tv = s.tri_verts + 3u * slot;
-  float3 v0 = xform_point(o2w, f3(tv[0])), v1 = xform_point(o2w, f3(tv[1])), v2 = xform_point(o2w, f3(tv[2]));
+  float3 v0, v1, v2;
+  load_triangle(tv, v0, v1, v2);
+  v0 = xform_point(o2w, v0);
+  v1 = xform_point(o2w, v1);
+  v2 = xform_point(o2w, v2);
   float3 ng = normalize(cross(v1 - v0, v2 - v0));
   const float4* tn = s.tri_normals + 3u * slot;
   float w0 = 1.0f - hit.y - hit.z;

@@ -151,7 +151,8 @@ OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, in
   constexpr int kTraceSteps = TraceSchedule<SCHED>::kSteps;
   constexpr uint32_t kRefillLanes = TraceSchedule<SCHED>::kRefillLanes;
   Traversal<STACK, ANY_HIT> tr;
-  int spill[OLC_SPILL];
+  int spill[OLC_SPILL + 1];
+  tr.init(smem, spill);
   uint32_t my = 0xffffffffu;
   bool exhausted = false;
   const uint32_t lt = (1u << lane_id()) - 1u;
@@ -181,7 +182,7 @@ OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, in
             float tmin, tmax;
             uint32_t root;
             load(my, o, d, tmin, tmax, root);
-            tr.begin(s, o, d, tmin, tmax, root, smem, spill);
+            tr.begin(o, d, tmin, tmax, root);
           }
         }
         if (base + take >= n) exhausted = true;
@@ -509,7 +510,11 @@ __global__ void __maxnreg__(ShadeRegisters<kMedia>::kCap) k_shade(ShadeArgs a) {
         Affine o2w{ir.o2w0, ir.o2w1, ir.o2w2};
         Affine w2o{ir.w2o0, ir.w2o1, ir.w2o2};
         const float4* tv = s.tri_verts + 3u * slot;
-        float3 v0 = xform_point(o2w, f3(tv[0])), v1 = xform_point(o2w, f3(tv[1])), v2 = xform_point(o2w, f3(tv[2]));
+        float3 v0, v1, v2;
+        load_triangle(tv, v0, v1, v2);
+        v0 = xform_point(o2w, v0);
+        v1 = xform_point(o2w, v1);
+        v2 = xform_point(o2w, v2);
         float3 e1 = v1 - v0, e2 = v2 - v0;
         float3 gcross = cross(e1, e2);
         float3 ng = normalize(gcross);
@@ -1017,44 +1022,59 @@ __global__ void k_camera_rays(const JobRec* __restrict__ job_ptr, uint32_t sampl
   }
 }
 
+// Closest hits of caller-supplied rays, with the wavefront's persistent
+// traversal.
 template <int STACK>
-__global__ void __launch_bounds__(256) k_trace_rays(SceneView s, uint32_t root, uint32_t n,
-                                                    const float* __restrict__ origins, const float* __restrict__ dirs,
-                                                    float t_min, uint32_t* inst_id, int32_t* prim, float* tout,
-                                                    float* bary, Counters* cnt) {
+__global__ void __maxnreg__(kTraceRegisters) k_trace_rays(SceneView s, uint32_t root_node, uint32_t n,
+                                                          const float* __restrict__ origins,
+                                                          const float* __restrict__ dirs, float t_min,
+                                                          uint32_t* inst_id, int32_t* prim, float* tout, float* bary,
+                                                          Counters* cnt) {
   extern __shared__ int smem_stack[];
   uint32_t err = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float3 o = f3(origins[3ull * i], origins[3ull * i + 1], origins[3ull * i + 2]);
-    float3 d = f3(dirs[3ull * i], dirs[3ull * i + 1], dirs[3ull * i + 2]);
-    HitResult hr;
-    bool hit = olc_traverse<STACK, false>(s, root, o, d, t_min, CUDART_INF_F, hr, smem_stack, err);
-    if (inst_id)
-      inst_id[i] = hit ? s.instances[owner_instance(s.instances, s.tri_owner, hr.instance, hr.slot)].instance_id
-                       : 0xffffffffu;
-    if (prim) prim[i] = hit ? (int32_t)hr.packed : -1;
-    if (tout) tout[i] = hit ? hr.t : CUDART_INF_F;
-    if (bary) {
-      bary[2ull * i] = hit ? hr.u : 0.0f;
-      bary[2ull * i + 1] = hit ? hr.v : 0.0f;
-    }
-  }
+  persistent_trace<STACK, false, 0>(
+      s, n, &cnt->closest_cursor[0], smem_stack,
+      [&](uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& root) {
+        o = f3(origins[3ull * i], origins[3ull * i + 1], origins[3ull * i + 2]);
+        d = f3(dirs[3ull * i], dirs[3ull * i + 1], dirs[3ull * i + 2]);
+        tmin = t_min;
+        tmax = CUDART_INF_F;
+        root = root_node;
+      },
+      [&](uint32_t i, const Traversal<STACK, false>& tr) {
+        const bool hit = tr.found();
+        if (inst_id)
+          inst_id[i] = hit ? s.instances[owner_instance(s.instances, s.tri_owner, tr.hit_inst, tr.hit_slot)].instance_id
+                           : 0xffffffffu;
+        if (prim) prim[i] = hit ? (int32_t)packed_index(s, tr.hit_inst, tr.hit_slot) : -1;
+        if (tout) tout[i] = hit ? tr.hit_t : CUDART_INF_F;
+        if (bary) {
+          bary[2ull * i] = hit ? tr.hit_u() : 0.0f;
+          bary[2ull * i + 1] = hit ? tr.hit_v() : 0.0f;
+        }
+      },
+      err);
   if (err) atomicAdd(&cnt->traversal_errors, 1u);
 }
 
 template <int STACK>
-__global__ void __launch_bounds__(256) k_occluded_rays(SceneView s, uint32_t root, uint32_t n,
-                                                       const float* __restrict__ origins,
-                                                       const float* __restrict__ dirs, float t_min,
-                                                       const float* __restrict__ t_max, uint8_t* occ, Counters* cnt) {
+__global__ void __maxnreg__(kTraceRegisters) k_occluded_rays(SceneView s, uint32_t root_node, uint32_t n,
+                                                             const float* __restrict__ origins,
+                                                             const float* __restrict__ dirs, float t_min,
+                                                             const float* __restrict__ t_max, uint8_t* occ,
+                                                             Counters* cnt) {
   extern __shared__ int smem_stack[];
   uint32_t err = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float3 o = f3(origins[3ull * i], origins[3ull * i + 1], origins[3ull * i + 2]);
-    float3 d = f3(dirs[3ull * i], dirs[3ull * i + 1], dirs[3ull * i + 2]);
-    HitResult hr;
-    occ[i] = olc_traverse<STACK, true>(s, root, o, d, t_min, t_max[i], hr, smem_stack, err) ? 1 : 0;
-  }
+  persistent_trace<STACK, true, 0>(
+      s, n, &cnt->shadow_cursor[0], smem_stack,
+      [&](uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& root) {
+        o = f3(origins[3ull * i], origins[3ull * i + 1], origins[3ull * i + 2]);
+        d = f3(dirs[3ull * i], dirs[3ull * i + 1], dirs[3ull * i + 2]);
+        tmin = t_min;
+        tmax = t_max[i];
+        root = root_node;
+      },
+      [&](uint32_t i, const Traversal<STACK, true>& tr) { occ[i] = tr.found() ? 1 : 0; }, err);
   if (err) atomicAdd(&cnt->traversal_errors, 1u);
 }
 
@@ -1222,7 +1242,7 @@ void launch_trace_rays(const LaunchShape& ls, const SceneView& s, uint32_t root,
                        Counters* cnt, cudaStream_t stream) {
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
-    uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>((n + kTraceThreads - 1) / kTraceThreads, ls.grid_trace));
+    const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
     k_trace_rays<D><<<grid, kTraceThreads, stack_bytes(D, kTraceThreads), stream>>>(s, root, n, origins, dirs, t_min,
                                                                                      inst_id, prim, t, bary, cnt);
   });
@@ -1234,7 +1254,7 @@ void launch_occluded_rays(const LaunchShape& ls, const SceneView& s, uint32_t ro
                           cudaStream_t stream) {
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
-    uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>((n + kTraceThreads - 1) / kTraceThreads, ls.grid_trace));
+    const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
     k_occluded_rays<D><<<grid, kTraceThreads, stack_bytes(D, kTraceThreads), stream>>>(s, root, n, origins, dirs,
                                                                                         t_min, t_max, occ, cnt);
   });

@@ -1,0 +1,57 @@
+"""Kernel edges on the device: sizes and shapes where a kernel's split, its
+shared stack or a dispatch rule can go wrong, against brute force, a library
+sort or the oracle."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import ordinarylight_b200 as ol
+from ordinarylight_b200 import CudaWavefrontRenderer, _native
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh_scene(vertices, indices, normal=(0.0, 0.0, 1.0)):
+    """A scene of one mesh (its own normals and tangents, so making it is quick)."""
+    scene = ol.Scene()
+    n = np.tile(np.asarray(normal, np.float32), (len(vertices), 1))
+    tangents = np.tile(np.float32([1.0, 0.0, 0.0, 1.0]), (len(vertices), 1))
+    mesh = scene.create_mesh(np.asarray(vertices, np.float32), np.asarray(indices, np.uint32),
+                             ol.Material(base_color=(0.5, 0.5, 0.5)), normals=n, tangents=tangents)
+    scene.add_instance(mesh)
+    return scene
+
+
+@pytest.mark.parametrize("stack_depth", [16, 24, 32])
+@pytest.mark.parametrize("rays", [1, 33, 5000, 40_000])
+def test_deep_stacks_and_every_ray_count(native_library, cuda_device, stack_depth, rays):
+    """20,000 parallel sheets: a ray through them meets all four boxes of every
+    node, so its stack (three entries a level) runs past 16 shared entries into
+    the overflow.  Half of the rays pass each sheet's box beside its triangle
+    and visit the whole tree.  Ray counts below and above one ray per warp."""
+    sheets = 20_000
+    z = np.arange(sheets, dtype=np.float32)
+    v = np.zeros((sheets, 3, 3), np.float32)
+    v[:, 1, 0] = v[:, 2, 1] = 1.0
+    v[:, :, 2] = z[:, None]
+    scene = _mesh_scene(v.reshape(-1, 3), np.arange(3 * sheets).reshape(-1, 3))
+    rng = np.random.default_rng(rays)
+    xy = rng.uniform(0.05, 0.45, (rays, 2))
+    outside = np.arange(rays) % 2 == 1
+    xy[outside] += 0.5                        # x + y > 1: in the box, off the triangle
+    start = rng.integers(-1, sheets - 1, rays) + 0.5
+    o = np.column_stack([xy, start]).astype(np.float32)
+    up = np.arange(rays) % 3 != 0
+    d = np.zeros((rays, 3), np.float32)
+    d[:, 2] = np.where(up, 1.0, -1.0)
+    first = np.where(up, np.ceil(start), np.floor(start)).astype(np.int64)
+    hit = ~outside & (first >= 0) & (first < sheets)
+    with CudaWavefrontRenderer(stack_depth=stack_depth) as r:
+        _inst, prim, t, _ = r.trace_closest(scene, o, d)
+        np.testing.assert_array_equal(prim, np.where(hit, first, -1))
+        np.testing.assert_array_equal(t, np.where(hit, 0.5, np.inf).astype(np.float32))
+        far = np.full(rays, 1e9, np.float32)
+        np.testing.assert_array_equal(r.trace_occluded(scene, o, d, far), hit)
+        np.testing.assert_array_equal(r.trace_occluded(scene, o, d, np.full(rays, 0.25, np.float32)), np.zeros(rays, bool))
