@@ -88,7 +88,8 @@ void morton_codes(const float4* centers, uint32_t n, uint32_t* bounds_scratch, u
 // Centres of triangle AABBs from a flat [n*9] array (tests).
 void triangle_centers_flat(const float* tri, uint32_t n, float4* lo, float4* hi, float4* centers,
                            cudaStream_t stream);
-// Stable LSD radix sort of pairs; result lands in keys/vals.
+// Stable LSD radix sort of pairs; result lands in keys/vals.  `hist` holds
+// radix_sort_hist_words(n) words, 16-byte aligned.
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt,
                       uint32_t* hist, uint32_t n, uint32_t key_bits, cudaStream_t stream);
 size_t radix_sort_hist_words(uint32_t n);

@@ -34,8 +34,10 @@
 namespace {
 
 constexpr uint32_t kNoAllocMaxPairs = 1u << 20;
-// ping-pong keys, ping-pong values, histogram (256 digits x blocks of 2048)
-constexpr size_t kNoAllocHistWords = 256u * ((kNoAllocMaxPairs + 2047u) / 2048u);
+// ping-pong keys, ping-pong values, histogram (256 digits x blocks of 2048,
+// and one total per 4,096 of those counts: radix_sort_hist_words)
+constexpr size_t kNoAllocCounts = 256u * ((kNoAllocMaxPairs + 2047u) / 2048u);
+constexpr size_t kNoAllocHistWords = kNoAllocCounts + (kNoAllocCounts + 4095u) / 4096u;
 constexpr size_t kNoAllocWords = 2u * kNoAllocMaxPairs + kNoAllocHistWords;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
@@ -99,6 +101,8 @@ extern "C" int olc_radix_sort_pairs_noalloc(uint32_t n, uint32_t key_bits, uint3
                                           std::to_string(n));
     if (n == 0) return OLC_OK;
     if (!keys || !values) throw olc::Error(OLC_ERR_VALUE, "keys and values are required");
+    if (olc::radix_sort_hist_words(n) > kNoAllocHistWords)
+      throw olc::Error(OLC_ERR_RUNTIME, "the sort's histogram does not fit the static scratch");
     uint32_t* scratch = scratch_on_current_device();
     uint32_t* keys_alt = scratch;
     uint32_t* vals_alt = scratch + kNoAllocMaxPairs;

@@ -81,3 +81,23 @@ def test_morton_cells_of_any_extent_build_a_valid_tree(native_library, cuda_devi
     if np.linalg.norm(extent) < 200:
         assert hit.mean() > 0.97
     assert np.all(t[hit] <= dist[hit] * (1 + 1e-4) + 0.05) or np.linalg.norm(extent) >= 200
+
+
+@pytest.mark.parametrize("n", [32_768, 32_769, 1_048_576, 2_097_153, 34_000_001])
+@pytest.mark.parametrize("bits", [8, 30])
+def test_radix_sort_across_scan_tiles(native_library, cuda_device, n, bits):
+    """Pair counts at which the digit histogram fills exactly one scan tile,
+    one more block, the static scratch's limit, and more tiles than the scan
+    of the tile totals takes in one pass: equal to a stable library sort."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    keys = torch.randint(0, 1 << bits, (n,), generator=g, device="cuda", dtype=torch.int64)
+    keys[::3] &= 0xFF   # many equal keys
+    k, v = keys.to(torch.int32), torch.arange(n, dtype=torch.int32, device="cuda")
+    want, order = torch.sort(keys, stable=True)
+    with CudaWavefrontRenderer() as r:
+        torch.cuda.synchronize()
+        _native.check(r._lib, r._ctx, r._lib.olc_radix_sort_pairs(r._ctx, n, bits, _native.ptr(k), _native.ptr(v)))
+        assert torch.equal(k.long(), want)
+        assert torch.equal(v.long(), order)
