@@ -203,76 +203,124 @@ OLC_D float3 rv_scattering(const RefVolumeView& V, const RefVolume& v, const Lig
   return result * f3(v.scat_color_aniso);
 }
 
-// Radiance gained and transmittance of the segment [0, t_max] of the ray.
+// Lanes that cross one ray together.  A ray's march is a chain of 50 to 100
+// steps, each some 250 instructions for two media, and a frame of this mode
+// has 30,000 to 100,000 such rays a bounce: one thread a ray left the SMs a
+// quarter full and waiting for the longest ray.  Eight lanes take eight
+// consecutive steps at once (and the eight volumes' scattering sources one
+// each); only the running transmittance is passed along in step order.
+// Two media, 115,200 / 44,009 / 30,510 rays at bounces 0 to 2 of a 320x180
+// frame of 2 samples: 427 -> 190 us for the three marches.
+constexpr uint32_t kRvLanes = 8;
+static_assert(kRvLanes == kMaxRefVolumes, "one lane computes one volume's interval and scattering source");
+
+// What the lanes of one ray share: the crossed intervals and scattering
+// sources by volume, and the sorted interval events.
+struct RvShared {
+  float en[kMaxRefVolumes], ex[kMaxRefVolumes];
+  float sx[kMaxRefVolumes], sy[kMaxRefVolumes], sz[kMaxRefVolumes];
+  float events[2 * kMaxRefVolumes];
+  uint32_t inside, num_events;
+};
+
+// Radiance gained and transmittance of the segment [0, t_max] of the ray,
+// for the kRvLanes lanes of `mask` (lane: this one's index among them).  Every
+// lane returns the transmittance; the radiance is the sum over the lanes.
 OLC_D void rv_integrate(const RefVolumeView& V, const LightRec* lights, uint32_t num_lights, float3 o, float3 d,
-                        float t_max, float3& radiance, float& transmittance) {
+                        float t_max, uint32_t mask, uint32_t lane, RvShared& sh, float3& radiance,
+                        float& transmittance) {
   radiance = f3(0.0f, 0.0f, 0.0f);
   transmittance = 1.0f;
-  float en[kMaxRefVolumes], ex[kMaxRefVolumes];
-  float3 source[kMaxRefVolumes];
-  uint32_t inside = 0;   // bit k: the ray crosses volume k
-  float events[2 * kMaxRefVolumes];
-  uint32_t ne = 0;
-  for (uint32_t k = 0; k < V.count; ++k) {
+  bool crossed = false;
+  if (lane < V.count) {
+    const RefVolume& v = V.vols[lane];
     float a, b;
-    if (!rv_box(V.vols[k], o, d, a, b)) continue;
-    b = fminf(b, t_max);
-    if (!(isfinite(a) && b > a)) continue;
-    en[k] = a;
-    ex[k] = b;
-    inside |= 1u << k;
-    const RefVolume& v = V.vols[k];
-    source[k] = f3(0.0f, 0.0f, 0.0f);
-    if (v.scattering_scale > 0.0f && num_lights > 0u) {
-      const float3 mid = o + d * (0.5f * (a + b));
-      const float4 rgba = rv_rgba(v, V.grid, V.lut, mid);
-      const float depth = rv_extinction(v, rgba.w) * (b - a);
-      source[k] = rv_scattering(V, v, lights, num_lights, mid, d, depth) * v.scattering_scale;
-    }
-    // events: sorted, without duplicates
-    for (float e : {a, b}) {
-      uint32_t pos = 0;
-      while (pos < ne && events[pos] < e) ++pos;
-      if (pos < ne && events[pos] == e) continue;
-      for (uint32_t q = ne; q > pos; --q) events[q] = events[q - 1];
-      events[pos] = e;
-      ++ne;
+    if (rv_box(v, o, d, a, b)) {
+      b = fminf(b, t_max);
+      crossed = isfinite(a) && b > a;
+      if (crossed) {
+        sh.en[lane] = a;
+        sh.ex[lane] = b;
+        float3 source = f3(0.0f, 0.0f, 0.0f);
+        if (v.scattering_scale > 0.0f && num_lights > 0u) {
+          const float3 mid = o + d * (0.5f * (a + b));
+          const float4 rgba = rv_rgba(v, V.grid, V.lut, mid);
+          const float depth = rv_extinction(v, rgba.w) * (b - a);
+          source = rv_scattering(V, v, lights, num_lights, mid, d, depth) * v.scattering_scale;
+        }
+        sh.sx[lane] = source.x;
+        sh.sy[lane] = source.y;
+        sh.sz[lane] = source.z;
+      }
     }
   }
+  const uint32_t first_lane = __ffs(mask) - 1u;
+  const uint32_t inside = __ballot_sync(mask, crossed) >> first_lane;   // bit k: the ray crosses volume k
   if (!inside) return;
+  if (lane == 0u) {
+    // events: sorted, without duplicates
+    uint32_t ne = 0;
+    for (uint32_t k = 0; k < V.count; ++k) {
+      if (!((inside >> k) & 1u)) continue;
+      for (int end = 0; end < 2; ++end) {
+        const float e = end ? sh.ex[k] : sh.en[k];
+        uint32_t pos = 0;
+        while (pos < ne && sh.events[pos] < e) ++pos;
+        if (pos < ne && sh.events[pos] == e) continue;
+        for (uint32_t q = ne; q > pos; --q) sh.events[q] = sh.events[q - 1];
+        sh.events[pos] = e;
+        ++ne;
+      }
+    }
+    sh.num_events = ne;
+  }
+  __syncwarp(mask);
+  const uint32_t ne = sh.num_events;
   float T = 1.0f;
   float3 L = f3(0.0f, 0.0f, 0.0f);
   for (uint32_t s = 0; s + 1 < ne && T >= 1e-4f; ++s) {
-    const float s0 = events[s], s1 = events[s + 1], mid = 0.5f * (s0 + s1);
+    const float s0 = sh.events[s], s1 = sh.events[s + 1], mid = 0.5f * (s0 + s1);
     uint32_t active = 0;
     float ref_step = CUDART_INF_F;
     for (uint32_t k = 0; k < V.count; ++k)
-      if (((inside >> k) & 1u) && en[k] <= mid && mid < ex[k]) {
+      if (((inside >> k) & 1u) && sh.en[k] <= mid && mid < sh.ex[k]) {
         active |= 1u << k;
         ref_step = fminf(ref_step, V.vols[k].step_size);
       }
     if (!active) continue;
     const uint32_t steps = min((uint32_t)ceilf((s1 - s0) / ref_step), kMaxRefSteps);
     const float dt = (s1 - s0) / (float)max(steps, 1u);
-    for (uint32_t i = 0; i < steps; ++i) {
-      const float3 p = o + d * (s0 + ((float)i + 0.5f) * dt);
-      float ext = 0.0f;
-      float3 emit = f3(0.0f, 0.0f, 0.0f), scat = f3(0.0f, 0.0f, 0.0f);
-      for (uint32_t k = 0; k < V.count; ++k) {
-        if (!((active >> k) & 1u)) continue;
-        const RefVolume& v = V.vols[k];
-        const float4 rgba = rv_rgba(v, V.grid, V.lut, p);
-        const float e = rv_extinction(v, rgba.w);
-        ext += e;
-        emit += f3(rgba.x, rgba.y, rgba.z) * (e * v.emission_scale);
-        scat += source[k] * e;
+    for (uint32_t first = 0; first < steps && T >= 1e-4f; first += kRvLanes) {
+      const uint32_t i = first + lane;
+      float alpha = 0.0f, ext = 0.0f;
+      float3 glow = f3(0.0f, 0.0f, 0.0f);
+      if (i < steps) {
+        const float3 p = o + d * (s0 + ((float)i + 0.5f) * dt);
+        float3 emit = f3(0.0f, 0.0f, 0.0f), scat = f3(0.0f, 0.0f, 0.0f);
+        for (uint32_t k = 0; k < V.count; ++k) {
+          if (!((active >> k) & 1u)) continue;
+          const RefVolume& v = V.vols[k];
+          const float4 rgba = rv_rgba(v, V.grid, V.lut, p);
+          const float e = rv_extinction(v, rgba.w);
+          ext += e;
+          emit += f3(rgba.x, rgba.y, rgba.z) * (e * v.emission_scale);
+          scat += f3(sh.sx[k], sh.sy[k], sh.sz[k]) * e;
+        }
+        if (ext > 1e-12f) {
+          alpha = 1.0f - expf(-ext * dt);
+          glow = emit + scat;
+        }
       }
-      if (ext > 1e-12f) {
-        const float alpha = 1.0f - expf(-ext * dt);
-        L += (emit + scat) * (T * alpha / ext);
-        T *= 1.0f - alpha;
+      // the transmittance in front of each step, multiplied in step order; a
+      // step behind the point where it falls below 1e-4 is not taken
+      const float pass = 1.0f - alpha;
+      float before = T;
+      for (uint32_t j = 0; j < kRvLanes; ++j) {
+        const float p = __shfl_sync(mask, pass, first_lane + j);
+        if (T >= 1e-4f) T *= p;
+        if (j + 1u == lane) before = T;
       }
-      if (T < 1e-4f) break;
+      if (before >= 1e-4f && alpha != 0.0f) L += glow * (before * alpha / ext);
     }
   }
   radiance = L;

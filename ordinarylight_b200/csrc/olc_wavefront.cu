@@ -869,13 +869,18 @@ __global__ void k_sort_scatter(RayQueue in, const uint32_t* __restrict__ count, 
 // shading: path radiance += throughput * volume radiance, throughput *=
 // volume transmittance (ReferencePathTracer.render_hdr,
 // renderers/reference/path_tracer.py:55-65; the march is in
-// olc_refvolume.cuh).  A grid-stride pass over the bounce's queue; rays of
-// other paths are skipped.
+// olc_refvolume.cuh).  kRvLanes lanes take a queue entry, in a grid-stride
+// pass; rays of other paths are skipped.
 __global__ void __launch_bounds__(128) k_ref_volumes(const JobRec* __restrict__ jobs, SceneView s, RayQueue q,
                                                      HitBuf h, PathState ps, const Counters* __restrict__ cnt,
                                                      uint32_t bounce) {
+  __shared__ RvShared shared[128 / kRvLanes];
   const uint32_t n = cnt->queue_count[bounce];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x % kRvLanes, group = threadIdx.x / kRvLanes;
+  const uint32_t mask = ((1u << kRvLanes) - 1u) << (lane_id() - lane);
+  RvShared& sh = shared[group];
+  const uint32_t groups = blockDim.x / kRvLanes;
+  for (uint32_t i = blockIdx.x * groups + group; i < n; i += gridDim.x * groups) {
     const uint32_t path = q.path[i];
     const uint4 meta = ps.meta[path];
     const JobRec& job = jobs[meta.w];
@@ -887,8 +892,14 @@ __global__ void __launch_bounds__(128) k_ref_volumes(const JobRec* __restrict__ 
     float3 rad;
     float T;
     rv_integrate(ref_volumes_of(sc), s.lights + sc.light_base, sc.num_lights, f3(q.origin_tmin[i]),
-                 f3(q.dir_root[i]), t_max, rad, T);
-    if (T == 1.0f && rad.x == 0.0f && rad.y == 0.0f && rad.z == 0.0f) continue;
+                 f3(q.dir_root[i]), t_max, mask, lane, sh, rad, T);
+    for (uint32_t off = kRvLanes / 2u; off > 0u; off >>= 1) {
+      rad.x += __shfl_xor_sync(mask, rad.x, off);
+      rad.y += __shfl_xor_sync(mask, rad.y, off);
+      rad.z += __shfl_xor_sync(mask, rad.z, off);
+    }
+    __syncwarp(mask);   // the next ray of these lanes rewrites sh
+    if (lane != 0u || (T == 1.0f && rad.x == 0.0f && rad.y == 0.0f && rad.z == 0.0f)) continue;
     const float4 tp = ps.throughput[path];
     const float4 r = ps.radiance[path];
     ps.radiance[path] = make_float4(r.x + tp.x * rad.x, r.y + tp.y * rad.y, r.z + tp.z * rad.z, r.w);

@@ -101,3 +101,36 @@ def test_radix_sort_across_scan_tiles(native_library, cuda_device, n, bits):
         _native.check(r._lib, r._ctx, r._lib.olc_radix_sort_pairs(r._ctx, n, bits, _native.ptr(k), _native.ptr(v)))
         assert torch.equal(k.long(), want)
         assert torch.equal(v.long(), order)
+
+
+@pytest.mark.parametrize("volumes,step,density", [(1, 0.4, 0.8), (1, 0.05, 60.0), (3, 0.031, 0.5), (8, 0.07, 0.3)])
+def test_volume_march_lane_groups(native_library, cuda_device, volumes, step, density):
+    """Marches of fewer steps than a ray's lanes, of step counts that are no
+    multiple of them, through media so dense that the transmittance ends the
+    march inside a group, and through as many overlapping volumes as a scene
+    takes: one camera segment per pixel against the oracle's float64 march."""
+    import parity_scenes
+    from oracle import reference_path_tracer as ref
+    from oracle import reference_volume
+    from ordinarylight_b200 import scenes
+
+    scene, camera = scenes.box_room()
+    tf = ol.Texture1D(np.array([[0.0, 0.0, 0.0, 0.0], [1.0, 0.5, 0.2, 0.3], [0.4, 0.6, 1.0, 0.9]], np.float32))
+    for k in range(volumes):
+        mat = ol.VolumeMaterial(transfer_function=tf, density_scale=density, emission_scale=0.5, step_size=step,
+                                scattering_scale=float(k % 2), scattering_orders=2)
+        scene.add_volume(parity_scenes._fbm_field(10 + k, 30 + k) + 0.05, mat,
+                         transform=ol.Transform.translation((-0.8 + 0.1 * k, 0.1 + 0.05 * k, -0.7)))
+    scene.add_light(ol.PointLight(position=(0.0, 1.7, -0.4), color=(1.0, 0.9, 0.7), intensity=2.0))
+    w, h = 23, 17
+    with CudaWavefrontRenderer(mode="reference_compatible", max_bounces=1) as r:
+        img = r.render_frame(scene, camera, w, h, samples=1)
+        o, d = r.camera_rays(camera, w, h, sample=0, frame_index=0)
+    tris, _colors, emissions = scene.triangles()
+    t, tri = ref.intersect(o.astype(np.float32), d.astype(np.float32), tris)
+    vols = scene.visible_volumes
+    entries, exits = reference_volume.intersect_unit_boxes(o, d, vols)
+    vol_rad, vol_t = reference_volume.integrate_volumes(vols, o, d, entries, exits, max_distance=t, lights=scene.lights)
+    surface = np.where((tri >= 0)[:, None], emissions[np.maximum(tri, 0)], ref.sky(d, scene.environment))
+    # float32 sums of at most 4,096 steps and an exit at transmittance 1e-4, as the ray-by-ray parity test
+    np.testing.assert_allclose(img[..., :3].reshape(-1, 3), vol_rad + vol_t[:, None] * surface, rtol=2e-3, atol=5e-5)
