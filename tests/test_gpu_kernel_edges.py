@@ -134,3 +134,37 @@ def test_volume_march_lane_groups(native_library, cuda_device, volumes, step, de
     surface = np.where((tri >= 0)[:, None], emissions[np.maximum(tri, 0)], ref.sky(d, scene.environment))
     # float32 sums of at most 4,096 steps and an exit at transmittance 1e-4, as the ray-by-ray parity test
     np.testing.assert_allclose(img[..., :3].reshape(-1, 3), vol_rad + vol_t[:, None] * surface, rtol=2e-3, atol=5e-5)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (1, 5), (2, 2), (7, 3), (64, 64)])
+@pytest.mark.parametrize("wrap", ["repeat", "clamp", "mirror"])
+@pytest.mark.parametrize("linear", [True, False])
+def test_texture_lookups_at_the_wrap_seams(native_library, cuda_device, size, wrap, linear):
+    """Coordinates on and one rounding step beside every whole and half
+    period, for sizes down to one texel and whole and fractional mip levels,
+    against the restated lookup."""
+    from oracle import textures as otex
+    from ordinarylight_b200.packing import pack_scene
+
+    rng = np.random.default_rng(size[0] * 10 + size[1])
+    px = rng.integers(0, 256, (size[1], size[0], 4), dtype=np.uint8)
+    scene = ol.Scene()
+    quad = np.float32([[-1, 0, -1], [-1, 0, 1], [1, 0, 1], [1, 0, -1]])
+    mesh = scene.create_mesh(quad, np.uint32([[0, 1, 2], [0, 2, 3]]),
+                             ol.Material(base_color_texture=ol.Texture(px, wrap, wrap, linear)),
+                             normals=np.tile(np.float32([0, 1, 0]), (4, 1)), texcoords=quad[:, [0, 2]])
+    scene.add_instance(mesh)
+    packed = pack_scene(scene)
+    marks = np.arange(-4, 5, dtype=np.float32) / 2
+    u = np.concatenate([marks, np.nextafter(marks, np.float32(9)), np.nextafter(marks, np.float32(-9)),
+                        rng.uniform(-3, 3, 200).astype(np.float32)])
+    uv = np.stack(np.meshgrid(u, u), -1).reshape(-1, 2).astype(np.float32)
+    fp = rng.choice(np.float32([0.0, 1.0 / max(size), 2.0 / max(size), 0.3, 5.0]), len(uv))
+    with CudaWavefrontRenderer() as r:
+        for srgb in (False, True):
+            got = r.sample_texture(scene, 0, uv, uv, fp, fp, srgb=srgb)
+            want = otex.sample_material_texture(packed.texture_words, packed.texture_bindings, 0, uv, uv, srgb, fp, fp)
+            # float32 blends (the device may fuse them); a texel coordinate that rounds across a texel's edge
+            # moves a nearest lookup to its neighbour, on under 1 in 1,000 of these points
+            off = np.abs(got - want).max(1) > 1e-5
+            assert off.mean() < (1e-6 if linear else 1e-3)
