@@ -239,6 +239,7 @@ struct RunPlan {
   uint32_t max_segments = 0;
   uint32_t max_count = 0;
   bool restir = false;               // some chunk runs ReSTIR
+  bool restir_textures = false;      // some chunk runs ReSTIR over textured surfaces
   bool chunk_reservoirs = false;     // some ReSTIR segment uses chunk-local reservoirs
 };
 
@@ -1309,6 +1310,7 @@ void plan_run(std::vector<QueuedJob*>& jobs, uint64_t cap, uint32_t max_chunks, 
     ch.count = (uint32_t)fill;
     ch.textures = takes.front().job->textured;
     plan.restir = plan.restir || ch.restir;
+    plan.restir_textures = plan.restir_textures || (ch.restir && ch.textures);
     plan.max_segments = std::max<uint32_t>(plan.max_segments, (uint32_t)ch.segs.size());
     plan.max_count = std::max<uint32_t>(plan.max_count, ch.count);
     plan.chunks.push_back(std::move(ch));
@@ -1494,7 +1496,8 @@ void record_run(olc_context* ctx, const RunPlan& plan, const RunBuffers& rb) {
         tl_mark(ctx, OLC_STAGE_SHADE, b, c);
       }
       launch_shade(ctx->ls, jobs, s, *qin, rb.hb, *qout, rb.sq[b & 1u], rb.ps, rb.cnt, b, ctx->capacity, rb.prod,
-                   restir, ch.textures, ch.media, b == 0 && !ch.ref_volumes, st);
+                   restir, restir && ch.textures ? ctx->restir.surfaces.as<float4>() : nullptr, ch.textures, ch.media,
+                   b == 0 && !ch.ref_volumes, st);
       tl_mark(ctx, OLC_STAGE_SHADE, b, c);
       // this bounce's shadow rays on the side stream: they read only their
       // queue and add only to the paths' shadow sums, so the later bounces'
@@ -1550,7 +1553,7 @@ std::vector<uint64_t> run_signature(const olc_context* ctx, const RunPlan& plan,
                         ctx->restir.res_a0.get(), ctx->restir.res_a1.get(), ctx->restir.res_a2.get(),
                         ctx->restir.res_b0.get(), ctx->restir.res_b1.get(), ctx->restir.res_b2.get(),
                         ctx->restir.hist0.get(), ctx->restir.hist1.get(), ctx->restir.hist2.get(),
-                        ctx->restir.selected.get(), ctx->restir.hit_list.get(), ctx->restir.hit_count.get(),
+                        ctx->restir.selected.get(), ctx->restir.surfaces.get(), ctx->restir.hit_list.get(), ctx->restir.hit_count.get(),
                         ctx->restir.pool0.get(), ctx->restir.pool1.get(), ctx->restir.pool2.get()})
     ptr(p);
   k.push_back(rb.stride);
@@ -1783,7 +1786,8 @@ void run_to_completion(olc_context* ctx, std::vector<QueuedJob*>& jobs, olc_rend
   plan_run(jobs, plan_capacity(ctx, jobs), 0xffffffffu, job_local, plan);
   if (plan.restir)
     restir_prepare(ctx->restir, job_local + (plan.chunk_reservoirs ? plan.max_count : 0),
-                   std::max<uint32_t>(plan.max_count, 1), (uint32_t)plan.chunks.size(), plan.max_segments);
+                   std::max<uint32_t>(plan.max_count, 1), (uint32_t)plan.chunks.size(), plan.max_segments,
+                   plan.restir_textures);
   execute_run(ctx, plan, stats);
 }
 
@@ -2016,7 +2020,7 @@ int olc_pool_info_get(const olc_context* ctx, olc_pool_info* info) {
                                 &ctx->sample_lum, &ctx->motion_prev, &ctx->restir.res_a0,
                                 &ctx->restir.res_a1, &ctx->restir.res_a2, &ctx->restir.res_b0, &ctx->restir.res_b1,
                                 &ctx->restir.res_b2, &ctx->restir.hist0, &ctx->restir.hist1, &ctx->restir.hist2,
-                                &ctx->restir.selected, &ctx->restir.hit_list})
+                                &ctx->restir.selected, &ctx->restir.surfaces, &ctx->restir.hit_list})
     wf += b->bytes();
   info->wavefront_bytes = wf;
   info->pixel_bytes = ctx->pixels.bytes();
@@ -2197,7 +2201,7 @@ int olc_serve_step(olc_context* ctx, uint64_t* done, uint32_t done_capacity, uin
       try {
         if (plan.restir)
           restir_prepare(ctx->restir, plan.max_count, std::max<uint32_t>(plan.max_count, 1),
-                         (uint32_t)plan.chunks.size(), plan.max_segments);
+                         (uint32_t)plan.chunks.size(), plan.max_segments, plan.restir_textures);
         launch_planned(ctx, sl, std::move(plan));
       } catch (...) {
         // the chunk's jobs hold partial samples of a failed chunk: drop them

@@ -212,6 +212,7 @@ struct PrimaryVertex {
   float3 p, n, view;
   SurfaceMat m;
   float depth;
+  float occlusion;
 };
 
 template <bool kTextures>
@@ -245,12 +246,14 @@ OLC_D PrimaryVertex primary_vertex(const SceneView& s, const RayQueue& q, const 
   const uint32_t owner = owner_instance(s.instances, s.tri_owner, inst, slot);
   const uint32_t mi = s.instances[owner].material;
   pv.m = load_material(s, mi);
+  pv.occlusion = 1.0f;
   const SceneRec& sc = s.scenes[scene];
   if (kTextures && sc.tex_words != nullptr) {
     const TexturedHit th = apply_textures(sc, mi - sc.material_base, slot, v0, v1, v2, o2w, w2o, tn, hit.y, hit.z,
                                           0.0f, ng, ns, pv.m);
     pv.m = th.m;
     ns = th.ns;
+    pv.occlusion = th.occlusion;
   }
   pv.n = entering ? ns : -ns;
   pv.view = -d;
@@ -258,10 +261,29 @@ OLC_D PrimaryVertex primary_vertex(const SceneView& s, const RayQueue& q, const 
   return pv;
 }
 
-template <bool kTextures>
-OLC_D Surface primary_surface(const SceneView& s, const RayQueue& q, const HitBuf& h, uint32_t i, uint32_t scene) {
-  const PrimaryVertex pv = primary_vertex<kTextures>(s, q, h, i, scene);
+// What the resampling target reads of a primary vertex.  A textured chunk's
+// initial pass (kRecord) leaves the textured surface in `surfaces`; its later
+// passes read it back.
+template <bool kTextures, bool kRecord>
+OLC_D Surface primary_surface(const SceneView& s, const RayQueue& q, const HitBuf& h, uint32_t i, uint32_t scene,
+                              float4* surfaces) {
   Surface su;
+  if (kTextures && !kRecord) {
+    const SurfaceRecord r = load_surface(surfaces, i);
+    const float4 hit = h.tuv_slot[i], dr = q.dir_root[i], ot = q.origin_tmin[i];
+    SurfaceMat m{};
+    m.base = r.base;
+    m.roughness = r.roughness;
+    m.metallic = r.metallic;
+    su.p = f3(ot) + f3(dr) * hit.x;
+    su.bsdf = prepare_bsdf(m, r.n, -f3(dr));
+    su.depth = hit.x;
+    return su;
+  }
+  const PrimaryVertex pv = primary_vertex<kTextures>(s, q, h, i, scene);
+  if (kTextures && kRecord)
+    store_surface(surfaces, i, SurfaceRecord{pv.m.base, pv.m.emission, pv.n, pv.m.roughness, pv.m.metallic,
+                                             pv.m.transmission, pv.occlusion});
   su.p = pv.p;
   su.bsdf = prepare_bsdf(pv.m, pv.n, pv.view);
   su.depth = pv.depth;
@@ -329,6 +351,7 @@ struct RestirArgs {
   uint32_t pass;
   uint4* selected;
   uint32_t finalize;
+  float4* surfaces;         // textured surfaces of the listed hits (textured chunks)
   const float4* pool0;      // light pool: kPoolSize entries per chunk segment
   const float4* pool1;
   const float4* pool2;
@@ -398,7 +421,7 @@ __global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_initial(Resti
     const JobRec& job = a.jobs[meta.w];
     const SceneRec& sc = s.scenes[job.scene];
     const uint64_t g = reservoir_index(job, meta.y, meta.x);
-    const Surface su = primary_surface<kTextures>(s, a.q, a.h, i, job.scene);
+    const Surface su = primary_surface<kTextures, true>(s, a.q, a.h, i, job.scene, a.surfaces);
     const uint32_t stamp = a.hdr->stamp;
     Res r{0xffffffffu, 0u, 0.0f, 0u, 0.0f};
     uint32_t rng = olc_bounce_state(olc_path_seed(meta.x, meta.y, job.frame), kRestirStream);
@@ -453,7 +476,7 @@ __global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_initial(Resti
 // wave, the eighth block per SM took its ReSTIR time from 1.495 to 1.468 ms
 // per 1080p instanced frame.
 template <bool kTextures>
-__global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_spatial(RestirArgs a) {
+__global__ void __launch_bounds__(128, 8) k_restir_spatial(RestirArgs a) {
   const SceneView& s = a.s;
   const uint32_t n = *a.hit_count;
   // warps take the hit list 32 entries at a time (one atomic per grab),
@@ -474,7 +497,7 @@ __global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_spatial(Resti
     const JobRec& job = a.jobs[meta.w];
     const uint64_t g = reservoir_index(job, meta.y, meta.x);
     const uint64_t stream_base = g - meta.x;
-    const Surface su = primary_surface<kTextures>(s, a.q, a.h, i, job.scene);
+    const Surface su = primary_surface<kTextures, false>(s, a.q, a.h, i, job.scene, a.surfaces);
     const uint32_t stamp = a.hdr->stamp;
     float d0;
     uint32_t n0, st0;
@@ -541,7 +564,8 @@ __global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_spatial(Resti
 
 }  // namespace
 
-void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32_t chunks, uint32_t segments) {
+void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32_t chunks, uint32_t segments,
+                    bool textures) {
   if (reservoirs > st.reservoirs) {
     // the history survives only if its buffers are kept
     for (DeviceBuffer* b : {&st.res_a0, &st.res_a1, &st.res_a2, &st.res_b0, &st.res_b1, &st.res_b2, &st.hist0,
@@ -561,6 +585,7 @@ void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32
     st.hit_list.allocate((size_t)slots * 4);
     st.slots = slots;
   }
+  if (textures) st.surfaces.ensure((size_t)st.slots * 64);
   if (!st.hit_count.get()) st.hit_count.allocate(32);
   if ((uint64_t)st.next_stamp + chunks >= 0xffffffffull) {
     // stamps would wrap: clear every stored stamp and start again at 1
@@ -594,6 +619,7 @@ const uint4* restir_run(RestirState& st, const olc_config& cfg, const LaunchShap
   a.hist1 = st.hist1.as<uint4>();
   a.hist2 = st.hist2.as<uint4>();
   a.selected = st.selected.as<uint4>();
+  a.surfaces = st.surfaces.as<float4>();
   a.out0 = st.res_a0.as<uint4>();
   a.out1 = st.res_a1.as<uint4>();
   a.out2 = st.res_a2.as<uint4>();
@@ -665,6 +691,7 @@ void restir_release(RestirState& st) {
   for (DeviceBuffer* b : {&st.pool0, &st.pool1, &st.pool2}) b->release();
   st.pool_segments = 0;
   st.hit_list.release();
+  st.surfaces.release();
   st.hit_count.release();
   st.reservoirs = 0;
   st.slots = 0;

@@ -14,6 +14,7 @@ struct RestirState {
   DeviceBuffer hist0, hist1, hist2;      // previous frame's final reservoirs
   DeviceBuffer selected;           // per path slot: light, bary, W
   DeviceBuffer pool0, pool1, pool2;  // light pool of each chunk segment (k_restir_pool)
+  DeviceBuffer surfaces;           // per path slot: textured surface of its primary hit (textured chunks)
   DeviceBuffer hit_list;           // path slots whose primary ray hit (ReSTIR jobs only)
   DeviceBuffer hit_count;
   uint64_t reservoirs = 0;         // reservoir capacity (pixel-samples of ReSTIR jobs)
@@ -34,7 +35,9 @@ struct RestirState {
 // pools for `segments` chunk segments, and reserve one stamp per chunk of the
 // run (chunk c of the run gets st.run_first + c; the caller stores it and the
 // history's stamp range in each chunk header).
-void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32_t chunks, uint32_t segments);
+// `textures`: some chunk resamples over textured surfaces.
+void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32_t chunks, uint32_t segments,
+                    bool textures);
 // Run initial RIS (+ temporal for jobs with history) + spatial reuse for one
 // chunk over the primary hits the bounce-0 traversal listed in hit_list /
 // hit_count; returns the per-path-slot selected sample buffer consumed by the

@@ -186,6 +186,30 @@ struct TexturedHit {
   float occlusion;
 };
 
+// Textured surface of a ReSTIR job's primary hit (four float4 per path slot):
+// the texture lookups and the normal map cost several times what the rest of
+// a resampling pass does, so the initial pass, which needs them first, leaves
+// what they give for the spatial passes and the bounce-0 shading.  The same
+// values they would compute: the footprint of a camera ray is 0 everywhere.
+// 64 bytes written and read twice against two more rounds of lookups: a
+// 960x540 frame of 2 samples 2.71 -> 2.48 ms.
+struct SurfaceRecord {
+  float3 base, emission, n;   // n: shading normal on the viewer's side
+  float roughness, metallic, transmission, occlusion;
+};
+OLC_D void store_surface(float4* rec, uint32_t path, const SurfaceRecord& r) {
+  float4* p = rec + 4ull * path;
+  p[0] = make_float4(r.base.x, r.base.y, r.base.z, r.roughness);
+  p[1] = make_float4(r.emission.x, r.emission.y, r.emission.z, r.metallic);
+  p[2] = make_float4(r.n.x, r.n.y, r.n.z, r.occlusion);
+  p[3] = make_float4(r.transmission, 0.0f, 0.0f, 0.0f);
+}
+OLC_D SurfaceRecord load_surface(const float4* rec, uint32_t path) {
+  const float4* p = rec + 4ull * path;
+  const float4 a = p[0], b = p[1], c = p[2];
+  return SurfaceRecord{f3(a), f3(b), f3(c), a.w, b.w, p[3].x, c.w};
+}
+
 // Apply the material's textures at a hit (applyMaterialTextures and the
 // normal map of wavefront_shade.comp:368-391): the material's base colour,
 // emission, transmission, roughness and metallic and the shading normal

@@ -298,6 +298,7 @@ struct ShadeArgs {
   uint32_t capacity;
   ProductPtrs prod;
   const uint4* restir;   // per-path selected light sample (bounce 0), or null
+  const float4* surfaces;   // textured surfaces of ReSTIR jobs' primary hits (textured chunks, bounce 0), or null
   uint32_t fresh;        // every path is at its camera vertex with its initial state (throughput 1,
                          // previous pdf 0, radiance 0), which then is not read back
 };
@@ -563,11 +564,23 @@ __global__ void __maxnreg__(ShadeRegisters<kMedia>::kCap) k_shade(ShadeArgs a) {
               cone_s = c.y;
               cone_w = c.x + t * c.y;
             }
-            const TexturedHit th = apply_textures(sc, orec.material - sc.material_base, slot, v0, v1, v2, o2w, w2o,
-                                                  tn, bu, bv, cone_w, ng, ns, m);
-            m = th.m;
-            ns = th.ns;
-            occlusion = th.occlusion;
+            if (a.surfaces != nullptr && job.restir) {
+              // resampling has looked the textures up already
+              const SurfaceRecord r = load_surface(a.surfaces, path);
+              m.base = r.base;
+              m.emission = r.emission;
+              m.roughness = r.roughness;
+              m.metallic = r.metallic;
+              m.transmission = r.transmission;
+              ns = entering ? r.n : -r.n;
+              occlusion = r.occlusion;
+            } else {
+              const TexturedHit th = apply_textures(sc, orec.material - sc.material_base, slot, v0, v1, v2, o2w, w2o,
+                                                    tn, bu, bv, cone_w, ng, ns, m);
+              m = th.m;
+              ns = th.ns;
+              occlusion = th.occlusion;
+            }
           }
           const float3 nrm = entering ? ns : -ns;
           // denoiser path signals (the secondary path state of
@@ -1165,7 +1178,7 @@ uint32_t resident_grid(const void* fn, uint32_t block, size_t smem, uint32_t max
 void launch_shade(const LaunchShape& ls, const JobRec* jobs, const SceneView& s, const RayQueue& qin,
                   const HitBuf& hits, const RayQueue& qout, const ShadowQueue& sq, const PathState& ps,
                   Counters* cnt, uint32_t bounce, uint32_t capacity, const ProductPtrs& prod, const uint4* restir,
-                  bool textures, bool media, bool fresh, cudaStream_t stream) {
+                  const float4* surfaces, bool textures, bool media, bool fresh, cudaStream_t stream) {
   ShadeArgs a;
   a.jobs = jobs;
   a.s = s;
@@ -1179,6 +1192,7 @@ void launch_shade(const LaunchShape& ls, const JobRec* jobs, const SceneView& s,
   a.capacity = capacity;
   a.prod = prod;
   a.restir = restir;
+  a.surfaces = surfaces;
   a.fresh = fresh ? 1u : 0u;
   auto launch = [&](auto kernel) {
     kernel<<<resident_grid((const void*)kernel, ls.trace_block, 0, ls.grid_shade), ls.trace_block, 0, stream>>>(a);
