@@ -47,10 +47,12 @@ thread_local std::string g_thread_error;
 // world-space triangles referenced by the TLAS, up to kFlattenMaxTotal baked
 // triangles per scene.
 constexpr uint32_t kFlattenMaxTriangles = 64;
-// Triangles per BLAS leaf.  One triangle per leaf: the parent's child box
-// then bounds exactly that triangle, so a ray tests a triangle only when it
-// enters its box (measured per 1080p frame against 2 / 3 / 4 / 8 per leaf:
-// traversal 12 % faster than 4 on the instanced scene, 22 % on the terrain).
+// Triangles per leaf of a BLAS's binary tree.  One triangle per leaf: the
+// parent's child box then bounds exactly that triangle, so a ray tests a
+// triangle only when it enters its box (measured per 1080p frame against
+// 2 / 3 / 4 / 8 for every leaf: traversal 12 % faster than 4 on the instanced
+// scene, 22 % on the terrain).  Where two triangles in one leaf cost less, the
+// BVH4 form joins them (plan_collapse in olc_bvh.cu).
 constexpr uint32_t kBlasLeafTriangles = 1;
 constexpr uint64_t kFlattenMaxTotal = 1ull << 24;
 constexpr size_t kMaxGraphs = 16;

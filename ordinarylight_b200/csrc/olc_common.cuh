@@ -129,7 +129,8 @@ OLC_HD float2 olc_camera_jitter(uint32_t pixel, uint32_t sample, uint32_t frame)
 //   a = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)
 //   b = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
 //   c = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
-//   d = (child0, child1, -, -)   child >= 0: node index; child < 0: leaf
+//   d = (child0, child1, w, -)   child >= 0: node index; child < 0: leaf;
+//       w: how the node is collapsed into BVH4 nodes (plan_collapse)
 struct __align__(16) BvhNode {
   float4 a, b, c;
   int4 d;
@@ -142,9 +143,9 @@ OLC_HD uint32_t olc_leaf_count(int ref) { return (((uint32_t)(~ref)) & 7u) + 1u;
 #define OLC_EMPTY_CHILD ((int)0x80000000)
 
 // BVH4 node, 128 bytes (one L2 line, seven 16-byte loads): up to four
-// descendants of BVH2 node i (its children, each internal one opened in turn
-// while the largest box still fits four slots; a leaf stands for itself),
-// stored at index i of a second array parallel to the BVH2 nodes.  Traversal
+// descendants of BVH2 node i (chosen by plan_collapse; a leaf stands for
+// itself and two triangles may share one), stored at index i of a second
+// array parallel to the BVH2 nodes.  Traversal
 // descends about two BVH2 levels per dependent fetch.  Child references keep
 // the BVH2 encoding, and an internal child's index is its BVH2 index, so
 // roots, instance records and leaves are shared by both forms.  Box slot k of

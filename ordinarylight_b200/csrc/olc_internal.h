@@ -78,6 +78,7 @@ struct BuildScratch {
   DeviceBuffer sorted_lo, sorted_hi; // float4 per leaf in sorted order
   DeviceBuffer left, right, first, last, parent, leaf_parent, flags;
   DeviceBuffer node_lo, node_hi;     // float4 per internal node
+  DeviceBuffer plan;                 // float4 per internal node: collapse costs and word
   size_t capacity = 0;
   void ensure(size_t n);
 };
@@ -139,7 +140,7 @@ uint32_t build_tlas(const float* object_to_world, const uint2* slot_ranges, uint
                     BvhNode* nodes, uint32_t node_base, cudaStream_t stream);
 
 // The BVH4 form (BvhNode4) of BVH2 nodes [begin, begin + count): wide[i]
-// holds up to four descendants of nodes[i] (greedy surface-area collapse).
+// holds up to four descendants of nodes[i] (as their collapse words say).
 // Run after every build or refit that wrote those nodes.
 void build_bvh4(const BvhNode* nodes, BvhNode4* wide, uint32_t begin, uint32_t count, cudaStream_t stream);
 

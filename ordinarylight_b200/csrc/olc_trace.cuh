@@ -5,8 +5,8 @@
 // nativeOccluded in ordinarylight/shaders/transport_v1/lighting.glsl).
 // * TLAS and BLAS nodes share one node pool; a TLAS leaf is one instance.
 //   Traversal reads the BVH4 form of the pool (BvhNode4: up to four
-//   descendants of a BVH2 node in one 128-byte line, collapsed greedily by
-//   surface area), so each dependent fetch descends about two levels of the
+//   descendants of a BVH2 node in one 128-byte line, collapsed at the least
+//   surface-area cost, with up to two triangles a leaf), so each dependent fetch descends about two levels of the
 //   binary hierarchy.  A ray picks each axis's near and far box planes once
 //   from its direction's signs, so the slab test needs no per-axis min/max.
 //   Entering an instance transforms the ray to object space (t is preserved

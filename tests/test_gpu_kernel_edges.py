@@ -168,3 +168,51 @@ def test_texture_lookups_at_the_wrap_seams(native_library, cuda_device, size, wr
             # moves a nearest lookup to its neighbour, on under 1 in 1,000 of these points
             off = np.abs(got - want).max(1) > 1e-5
             assert off.mean() < (1e-6 if linear else 1e-3)
+
+
+@pytest.mark.parametrize("triangles", [65, 66, 67, 131_072, 131_073])
+@pytest.mark.parametrize("layout", ["soup", "twins", "line"])
+def test_planned_collapse_keeps_every_triangle(native_library, cuda_device, triangles, layout):
+    """BVH4 nodes and two-triangle leaves planned by the host's and the device's
+    builder (up to and above 131,072 triangles), with odd counts, coincident
+    triangles (every hit a tie between two) and boxes of zero area: the tree
+    validates and hits are the oracle's; visibility agrees with them."""
+    from oracle import production
+
+    rng = np.random.default_rng(triangles)
+    n = triangles
+    if layout == "line":      # triangles in the plane z = 0, in a row: flat boxes
+        c = np.zeros((n, 3))
+        c[:, 0] = np.arange(n)
+        v = c[:, None, :] + np.array([[0.0, 0.0, 0.0], [0.75, 0.0, 0.0], [0.0, 0.75, 0.0]])
+    else:
+        c = rng.uniform(-20.0, 20.0, (n, 3))
+        v = c[:, None, :] + rng.uniform(-0.4, 0.4, (n, 3, 3)) * (8.0 if n < 100 else 1.0)
+        if layout == "twins":
+            v[1::2] = v[0:n - 1:2][:len(v[1::2])]
+    v = v.astype(np.float32)
+    scene = _mesh_scene(v.reshape(-1, 3), np.arange(3 * n).reshape(-1, 3))
+    rays = 4000
+    aim = rng.integers(0, n, rays)
+    target = (v[aim].astype(np.float64) * rng.dirichlet((2, 2, 2), rays)[:, :, None]).sum(1)
+    away = rng.normal(size=(rays, 3))
+    away[:, 2] += np.copysign(0.5, away[:, 2])
+    o = (target + 3.0 * away).astype(np.float32)
+    d = target - o
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    with CudaWavefrontRenderer() as r:
+        assert r.validate_bvh(scene) == 0
+        _inst, prim, t, _ = r.trace_closest(scene, o, d, t_min=1e-4)
+        hit = prim >= 0
+        far = np.where(hit, t * np.float32(1.001) + np.float32(1e-3), np.float32(1e9)).astype(np.float32)
+        seen = r.trace_occluded(scene, o, d, far)
+        np.testing.assert_array_equal(seen, hit)
+    want, want_t = production.trace(scene, o, d, t_min=1e-4)
+    assert hit.mean() > 0.9
+    # the same triangle (either of two coincident ones from the oracle), or one at the same distance within rounding
+    same = (prim >> 1 == want >> 1) if layout == "twins" else (prim == want)
+    gap = np.abs(np.where(hit, t, 0.0) - np.where(want >= 0, want_t, 0.0))
+    assert np.all(same | (hit & (want >= 0) & (gap <= 4e-6 * np.abs(np.where(hit, t, 1.0)))))
+    assert same.mean() > 0.995
+    if layout == "twins":     # of two coincident triangles the lower index is reported
+        assert np.all(prim[hit & (prim < n - n % 2)] % 2 == 0)
