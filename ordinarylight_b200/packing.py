@@ -21,6 +21,7 @@ import math
 import numpy as np
 
 from . import _native
+from .scene import Scene, emission_luminance, emissive_weight, triangle_areas
 
 _LUMINANCE = np.array((0.2126, 0.7152, 0.0722), np.float64)
 
@@ -269,39 +270,40 @@ def emitter_records(scene):
     """Emissive triangles with a power CDF: the records and probabilities of
     Scene.emissive_triangle_data (scene/_core.py:2637-2691), computed with
     array operations.  Returns (records [n, 20] float32, total weight)."""
-    chunks, weights, sided = [], [], []
-    for mesh in scene.visible_meshes:
-        emission = np.asarray(mesh.material.emission, np.float32)
-        if not np.any(emission > 0.0) or not len(mesh.indices):
-            continue
-        tris = mesh.world_vertices[mesh.indices]
-        area = 0.5 * np.linalg.norm(np.cross(tris[:, 1] - tris[:, 0], tris[:, 2] - tris[:, 0]), axis=1)
-        keep = area > 1e-12
-        if not np.any(keep):
-            continue
-        tris, area = tris[keep], area[keep]
-        rec = np.zeros((len(tris), 20), np.float32)
-        rec[:, 0:3] = tris[:, 0]
-        rec[:, 4:7] = tris[:, 1]
-        rec[:, 8:11] = tris[:, 2]
-        rec[:, 12:15] = emission
-        rec[:, 15] = area
-        chunks.append(rec)
-        weights.append(area.astype(np.float64) * float(np.dot(emission.astype(np.float64), _LUMINANCE)))
-        sided.append(np.full(len(tris), 1.0 if getattr(mesh.material, "emission_two_sided", False) else 0.0,
-                             np.float32))
-    if not chunks:
+    lit = [m for m in scene.visible_meshes
+           if np.any(np.asarray(m.material.emission, np.float32) > 0.0) or emission_luminance(m.material) > 0.0]
+    parts = [m.world_vertices[m.indices] for m in lit]
+    areas = triangle_areas(parts)
+    sources = [(m, t, a) for m, t, a in zip(lit, parts, areas)
+               if len(t) and np.any(np.asarray(m.material.emission, np.float32) > 0.0)]
+    if not sources:
         return np.zeros((0, 20), np.float32), 0.0
-    rec = np.concatenate(chunks)
-    w = np.concatenate(weights)
+    counts = [len(t) for _m, t, _a in sources]
+    emission = np.asarray([m.material.emission for m, _t, _a in sources], np.float32)
+    lum = [float(np.dot(e, _LUMINANCE)) for e in emission.astype(np.float64)]
+    sided = [1.0 if getattr(m.material, "emission_two_sided", False) else 0.0 for m, _t, _a in sources]
+    area = np.concatenate([a for _m, _t, a in sources])
+    keep = area > 1e-12
+    if not np.any(keep):
+        return np.zeros((0, 20), np.float32), 0.0
+    tris, area = np.concatenate([t for _m, t, _a in sources])[keep], area[keep]
+    rec = np.zeros((len(tris), 20), np.float32)
+    rec[:, 0:3] = tris[:, 0]
+    rec[:, 4:7] = tris[:, 1]
+    rec[:, 8:11] = tris[:, 2]
+    rec[:, 12:15] = np.repeat(emission, counts, axis=0)[keep]
+    rec[:, 15] = area
+    w = area.astype(np.float64) * np.repeat(lum, counts)[keep]
     total = float(w.sum())
     prob = w / total if total > 0.0 else np.full(len(w), 1.0 / len(w))
     cdf = np.cumsum(prob)
     cdf[-1] = 1.0
     rec[:, 16] = cdf.astype(np.float32)
     rec[:, 17] = prob.astype(np.float32)
-    rec[:, 18] = np.concatenate(sided)
-    return rec, float(scene.emissive_light_weight) if hasattr(scene, "emissive_light_weight") else total
+    rec[:, 18] = np.repeat(np.asarray(sided, np.float32), counts)[keep]
+    if getattr(type(scene), "emissive_light_weight", None) is Scene.emissive_light_weight:
+        return rec, emissive_weight(lit, areas)   # the property's own sum, over the areas at hand
+    return rec, float(getattr(scene, "emissive_light_weight", total))
 
 
 def light_records(scene) -> np.ndarray:
