@@ -257,6 +257,7 @@ OLC_D void rv_integrate(const RefVolumeView& V, const LightRec* lights, uint32_t
   const uint32_t first_lane = __ffs(mask) - 1u;
   const uint32_t inside = __ballot_sync(mask, crossed) >> first_lane;   // bit k: the ray crosses volume k
   if (!inside) return;
+  __syncwarp(mask);   // a vote orders no memory: lane 0 reads what the other lanes have stored
   if (lane == 0u) {
     // events: sorted, without duplicates
     uint32_t ne = 0;

@@ -136,6 +136,43 @@ def test_volume_march_lane_groups(native_library, cuda_device, volumes, step, de
     np.testing.assert_allclose(img[..., :3].reshape(-1, 3), vol_rad + vol_t[:, None] * surface, rtol=2e-3, atol=5e-5)
 
 
+def test_volume_march_lanes_take_several_rays(native_library, cuda_device):
+    """More rays (96,000) than a full grid has lane groups (148 SMs x 12
+    blocks x 16), so every group marches several, which cross different ones
+    of eight scattered volumes: a group's intervals and sources of one ray
+    must not reach the next.  600 pixels against the oracle's float64 march."""
+    import parity_scenes
+    from oracle import reference_path_tracer as ref
+    from oracle import reference_volume
+    from ordinarylight_b200 import scenes
+
+    scene, camera = scenes.box_room()
+    tf = ol.Texture1D(np.array([[0.0, 0.0, 0.0, 0.0], [1.0, 0.5, 0.2, 0.3], [0.4, 0.6, 1.0, 0.9]], np.float32))
+    for k in range(8):
+        mat = ol.VolumeMaterial(transfer_function=tf, density_scale=0.9, emission_scale=0.3 * k, step_size=0.06,
+                                scattering_scale=float(k % 2), scattering_orders=1)
+        scene.add_volume(parity_scenes._fbm_field(10 + k, 40 + k) + 0.05, mat,
+                         transform=ol.Transform.translation((-0.9 + 0.55 * (k % 4), 0.1 + 0.9 * (k // 4), -0.8 + 0.2 * (k % 3)))
+                         @ ol.Transform.scale(0.7))
+    scene.add_light(ol.PointLight(position=(0.0, 1.7, -0.4), color=(1.0, 0.9, 0.7), intensity=2.0))
+    w, h = 320, 300
+    with CudaWavefrontRenderer(mode="reference_compatible", max_bounces=1) as r:
+        img = r.render_frame(scene, camera, w, h, samples=1)[..., :3].reshape(-1, 3)
+        o, d = r.camera_rays(camera, w, h, sample=0, frame_index=0)
+    pick = np.random.default_rng(4).choice(w * h, 600, replace=False)
+    o, d = o[pick], d[pick]
+    tris, _colors, emissions = scene.triangles()
+    t, tri = ref.intersect(o.astype(np.float32), d.astype(np.float32), tris)
+    vols = scene.visible_volumes
+    entries, exits = reference_volume.intersect_unit_boxes(o, d, vols)
+    crossed = (exits > np.maximum(entries, 0.0)).sum(0)
+    assert len(set(crossed.tolist())) >= 3      # rays of the picture cross none, one and several of the volumes
+    vol_rad, vol_t = reference_volume.integrate_volumes(vols, o, d, entries, exits, max_distance=t, lights=scene.lights)
+    surface = np.where((tri >= 0)[:, None], emissions[np.maximum(tri, 0)], ref.sky(d, scene.environment))
+    # as the march above: float32 sums and an exit at transmittance 1e-4
+    np.testing.assert_allclose(img[pick], vol_rad + vol_t[:, None] * surface, rtol=2e-3, atol=5e-5)
+
+
 @pytest.mark.parametrize("size", [(1, 1), (1, 5), (2, 2), (7, 3), (64, 64)])
 @pytest.mark.parametrize("wrap", ["repeat", "clamp", "mirror"])
 @pytest.mark.parametrize("linear", [True, False])
