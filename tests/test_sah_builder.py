@@ -162,3 +162,21 @@ def test_denormal_close_and_non_finite_centroids_stay_in_bounds(harness):
     lo2[7, 1] = np.nan
     m, child, boxes, order = _build(harness, lo2, hi2)
     assert m == n - 1 and sorted(order.tolist()) == list(range(n))
+
+
+@pytest.mark.parametrize("n", [64, 65, 66, 127, 700])
+@pytest.mark.parametrize("layout", ["soup", "plane", "line", "far"])
+def test_child_boxes_from_bins_are_their_primitives_boxes(harness, n, layout):
+    """Up to 64 primitives a node's child boxes come from the primitives,
+    above that from the bins: exact unions either way, also where one or two
+    axes cannot be binned, and beside primitives at infinity (whose node's
+    boxes compare with theirs)."""
+    rng = np.random.default_rng(n)
+    lo, hi = _triangle_boxes(rng, n)
+    if layout == "plane":
+        lo[:, 1] = hi[:, 1] = 3.0
+    elif layout == "line":
+        lo[:, 1:] = hi[:, 1:] = -1.0
+    elif layout == "far":
+        lo[::9, 0], hi[::9, 0] = -np.inf, np.inf      # NaN centroids: no bin scale is usable on that axis
+    _check_tree(lo, hi, *_build(harness, lo, hi))
