@@ -550,7 +550,9 @@ OLC_API int olc_trace_closest(olc_context* ctx, uint32_t n, const float* origins
                       uint32_t* instance_id, int32_t* primitive, float* t,
                       float* barycentrics);
 
-/* Occlusion of n rays on (t_min, t_max[i]): occluded[i] = 1 if any hit. */
+/* Occlusion of n rays on (t_min, t_max[i]): occluded[i] = 1 if any hit.
+ * Either query fails with OLC_ERR_RUNTIME where some ray's traversal stack
+ * overflowed or its step budget ran out. */
 OLC_API int olc_trace_occluded(olc_context* ctx, uint32_t n, const float* origins,
                        const float* directions, float t_min,
                        const float* t_max, uint8_t* occluded);

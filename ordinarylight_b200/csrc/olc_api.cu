@@ -1834,6 +1834,16 @@ bool same_camera(const JobRec& a, const JobRec& b) {
          same(a.cam_up, b.cam_up) && a.projection == b.projection;
 }
 
+// Wait for the ray query in flight; a ray whose stack overflowed or whose step
+// budget ran out has no answer.
+void finish_query(olc_context* ctx) {
+  uint32_t errors = 0;
+  OLC_CUDA(cudaMemcpyAsync(&errors, &ctx->counters.as<Counters>()->traversal_errors, sizeof(errors),
+                           cudaMemcpyDeviceToHost, ctx->stream));
+  OLC_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (errors) throw Error(OLC_ERR_RUNTIME, "traversal stack overflow");
+}
+
 }  // namespace
 
 namespace olc {
@@ -2471,10 +2481,7 @@ int olc_trace_closest(olc_context* ctx, uint32_t n, const float* origins, const 
     OLC_CUDA(cudaMemsetAsync(ctx->counters.get(), 0, sizeof(Counters), ctx->stream));
     launch_trace_rays(ctx->ls, pool_view(ctx), rs.rec.tlas_root, n, origins, directions, t_min, instance_id,
                       primitive, t, barycentrics, ctx->counters.as<Counters>(), ctx->stream);
-    Counters h;
-    OLC_CUDA(cudaMemcpyAsync(&h, ctx->counters.get(), sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
-    OLC_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (h.traversal_errors) throw Error(OLC_ERR_RUNTIME, "traversal stack overflow");
+    finish_query(ctx);
   });
 }
 
@@ -2489,7 +2496,7 @@ int olc_trace_occluded(olc_context* ctx, uint32_t n, const float* origins, const
     OLC_CUDA(cudaMemsetAsync(ctx->counters.get(), 0, sizeof(Counters), ctx->stream));
     launch_occluded_rays(ctx->ls, pool_view(ctx), rs.rec.tlas_root, n, origins, directions, t_min, t_max, occluded,
                          ctx->counters.as<Counters>(), ctx->stream);
-    OLC_CUDA(cudaStreamSynchronize(ctx->stream));
+    finish_query(ctx);
   });
 }
 

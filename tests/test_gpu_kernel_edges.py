@@ -57,6 +57,38 @@ def test_deep_stacks_and_every_ray_count(native_library, cuda_device, stack_dept
         np.testing.assert_array_equal(r.trace_occluded(scene, o, d, np.full(rays, 0.25, np.float32)), np.zeros(rays, bool))
 
 
+@pytest.mark.parametrize("instances,answered", [(100, True), (210, False)])
+def test_rays_past_the_step_budget_are_errors_in_both_queries(native_library, cuda_device, instances, answered):
+    """A ray beside the triangles of 20,000 sheets visits every node and leaf
+    of the mesh, 20,000 to 26,700 steps, in each of its coincident instances: 100
+    stay within the 4,194,304 steps a ray may take and 210 do not.  Neither
+    query may answer for a ray that it did not finish."""
+    sheets = 20_000
+    v = np.zeros((sheets, 3, 3), np.float32)
+    v[:, 1, 0] = v[:, 2, 1] = 1.0
+    v[:, :, 2] = np.arange(sheets, dtype=np.float32)[:, None]
+    scene = ol.Scene()
+    vertices = v.reshape(-1, 3)
+    mesh = scene.create_mesh(vertices, np.arange(3 * sheets).reshape(-1, 3), ol.Material(),
+                             normals=np.tile(np.float32([0.0, 0.0, 1.0]), (len(vertices), 1)),
+                             tangents=np.tile(np.float32([1.0, 0.0, 0.0, 1.0]), (len(vertices), 1)))
+    scene.add_instances(mesh, [ol.Transform.translation((0.0, 0.0, 0.0))] * instances)
+    o = np.float32([[0.75, 0.75, -1.0]])
+    d = np.float32([[0.0, 0.0, 1.0]])
+    far = np.full(1, 1e9, np.float32)
+    with CudaWavefrontRenderer() as r:
+        if answered:
+            assert r.trace_closest(scene, o, d)[1][0] == -1
+            assert not r.trace_occluded(scene, o, d, far)[0]
+        else:
+            with pytest.raises(RuntimeError, match="traversal"):
+                r.trace_closest(scene, o, d)
+            with pytest.raises(RuntimeError, match="traversal"):
+                r.trace_occluded(scene, o, d, far)
+            # the next query is answered
+            assert r.trace_closest(scene, np.float32([[0.25, 0.25, -1.0]]), d)[2][0] == 1.0
+
+
 @pytest.mark.parametrize("extent", [(100.0, 1.0, 100.0), (0.0, 5.0, 1000.0), (1e-3, 1.0, 1e3), (0.0, 0.0, 0.0)])
 def test_morton_cells_of_any_extent_build_a_valid_tree(native_library, cuda_device, extent):
     """Meshes above the host builder's limit whose extents differ by up to
