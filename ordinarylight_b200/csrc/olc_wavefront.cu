@@ -200,6 +200,7 @@ OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, in
 // state without spilling (the world ray and the hit's barycentrics live in
 // shared memory), so eight blocks of 128 threads stay resident per SM.
 constexpr int kTraceRegisters = 64;
+constexpr uint32_t kTraceResidentThreads = 65536 / kTraceRegisters;
 
 // kCamera: bounce 0, whose rays the kernel generates itself (the chunk's
 // paths in order, `cam` their jobs and path records) and whose primary hits
@@ -1116,6 +1117,34 @@ inline size_t stack_bytes(uint32_t depth, uint32_t threads) {
   return (size_t)(d + OLC_RAY_SAVE) * threads * sizeof(int);
 }
 
+// Launch a traversal kernel with shared memory for as many blocks as the
+// registers let an SM hold (1,024 threads' worth) and no more: the rest of the
+// SM's 256 KB is its L1 cache, and traversal is bound by the latency of its
+// node and triangle loads.  The largest carve-out had left the L1 28 KB; with
+// 39 words a thread (24 stack entries) eight blocks of 128 threads take 164 KB.
+// Terrain 11.19 -> 10.78 ms, 1080p instanced frame 6.48 -> 6.38 ms, textured
+// 2.38 -> 2.35 ms.  The driver takes the next configuration above the
+// percentage, which is rounded down.  It goes with the launch because the
+// block size does: sixteen blocks of 64 threads need 172 KB (with 64 threads
+// and the 164 KB of 128: 1080p frame 6.25 -> 6.22 ms, terrain 10.51 -> 10.39).
+template <class... Params, class... Args>
+void launch_traversal(void (*kernel)(Params...), uint32_t grid, uint32_t block, uint32_t depth, cudaStream_t stream,
+                      Args... args) {
+  const size_t smem = stack_bytes(depth, block);
+  const size_t resident = kTraceResidentThreads / block * (smem + 1024u);   // 1 KB a block is the driver's
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attr.val.sharedMemCarveout = (unsigned)std::min<size_t>(100u, resident * 100u / (228u * 1024u));
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(block);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  OLC_CUDA(cudaLaunchKernelEx(&config, kernel, args...));
+}
+
 }  // namespace
 
 void launch_trace_closest(const LaunchShape& ls, const SceneView& s, const RayQueue& q, const HitBuf& h,
@@ -1123,17 +1152,16 @@ void launch_trace_closest(const LaunchShape& ls, const SceneView& s, const RayQu
                           cudaStream_t stream) {
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
-    const size_t smem = stack_bytes(D, ls.trace_block);
     // camera rays come in 8x4-pixel tiles: a warp keeps its 32 coherent rays
     // to the end instead of refilling lanes with rays of other tiles
     if (cam != nullptr)
-      k_trace_closest<D, 1, true><<<ls.grid_trace, ls.trace_block, smem, stream>>>(s, q, h, cnt, 0u, hl, *cam);
+      launch_traversal(k_trace_closest<D, 1, true>, ls.grid_trace, ls.trace_block, D, stream, s, q, h, cnt, 0u, hl, *cam);
     else if (ls.scheduler == 1)
-      k_trace_closest<D, 1, false><<<ls.grid_trace, ls.trace_block, smem, stream>>>(s, q, h, cnt, bounce,
-                                                                                    HitListOut{}, CameraPaths{});
+      launch_traversal(k_trace_closest<D, 1, false>, ls.grid_trace, ls.trace_block, D, stream, s, q, h, cnt, bounce,
+                       HitListOut{}, CameraPaths{});
     else
-      k_trace_closest<D, 0, false><<<ls.grid_trace, ls.trace_block, smem, stream>>>(s, q, h, cnt, bounce,
-                                                                                    HitListOut{}, CameraPaths{});
+      launch_traversal(k_trace_closest<D, 0, false>, ls.grid_trace, ls.trace_block, D, stream, s, q, h, cnt, bounce,
+                       HitListOut{}, CameraPaths{});
   });
   OLC_LAUNCH_CHECK("k_trace_closest");
 }
@@ -1143,11 +1171,9 @@ void launch_trace_shadow(const LaunchShape& ls, const SceneView& s, const Shadow
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
     if (ls.scheduler == 1)
-      k_trace_shadow<D, 1><<<ls.grid_trace, ls.trace_block, stack_bytes(D, ls.trace_block), stream>>>(s, sq, ps, cnt,
-                                                                                                       bounce);
+      launch_traversal(k_trace_shadow<D, 1>, ls.grid_trace, ls.trace_block, D, stream, s, sq, ps, cnt, bounce);
     else
-      k_trace_shadow<D, 0><<<ls.grid_trace, ls.trace_block, stack_bytes(D, ls.trace_block), stream>>>(s, sq, ps, cnt,
-                                                                                                       bounce);
+      launch_traversal(k_trace_shadow<D, 0>, ls.grid_trace, ls.trace_block, D, stream, s, sq, ps, cnt, bounce);
   });
   OLC_LAUNCH_CHECK("k_trace_shadow");
 }
@@ -1268,8 +1294,8 @@ void launch_trace_rays(const LaunchShape& ls, const SceneView& s, uint32_t root,
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
     const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
-    k_trace_rays<D><<<grid, kTraceThreads, stack_bytes(D, kTraceThreads), stream>>>(s, root, n, origins, dirs, t_min,
-                                                                                     inst_id, prim, t, bary, cnt);
+    launch_traversal(k_trace_rays<D>, grid, kTraceThreads, D, stream, s, root, n, origins, dirs, t_min, inst_id, prim, t,
+                     bary, cnt);
   });
   OLC_LAUNCH_CHECK("k_trace_rays");
 }
@@ -1280,50 +1306,38 @@ void launch_occluded_rays(const LaunchShape& ls, const SceneView& s, uint32_t ro
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
     const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
-    k_occluded_rays<D><<<grid, kTraceThreads, stack_bytes(D, kTraceThreads), stream>>>(s, root, n, origins, dirs,
-                                                                                        t_min, t_max, occ, cnt);
+    launch_traversal(k_occluded_rays<D>, grid, kTraceThreads, D, stream, s, root, n, origins, dirs, t_min, t_max, occ,
+                     cnt);
   });
   OLC_LAUNCH_CHECK("k_occluded_rays");
 }
 
 void configure_trace_kernels() {
-  // Shared memory for as many blocks as the registers let an SM hold (eight of
-  // 128 threads) and no more: the rest of the SM's 256 KB is its L1 cache, and
-  // traversal is bound by the latency of its node and triangle loads.  The
-  // largest carve-out had left the L1 28 KB; with 39 words a thread (24 stack
-  // entries) eight blocks take 164 KB.  Terrain 11.19 -> 10.78 ms, 1080p
-  // instanced frame 6.48 -> 6.38 ms, textured 2.38 -> 2.35 ms.
-  // The percentage is rounded down: the driver takes the next configuration
-  // above it.  The dynamic limit allows the largest launch's stacks (32
-  // entries, 256 threads: above the 48 KB that needs no opt-in).
+  // The dynamic limit allows the largest launch's stacks (32 entries, 256
+  // threads: above the 48 KB that needs no opt-in).
   const int most = (int)stack_bytes(32, 256);
-  auto prefer = [most](const void* fn, int depth) {
-    const size_t resident = 8u * (stack_bytes((uint32_t)depth, kTraceThreads) + 1024u);   // 1 KB a block is the driver's
-    const int percent = (int)std::min<size_t>(100u, resident * 100u / (228u * 1024u));
-    cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  };
-  prefer((const void*)k_trace_closest<16, 0, false>, 16);
-  prefer((const void*)k_trace_closest<24, 0, false>, 24);
-  prefer((const void*)k_trace_closest<32, 0, false>, 32);
-  prefer((const void*)k_trace_closest<16, 1, true>, 16);
-  prefer((const void*)k_trace_closest<24, 1, true>, 24);
-  prefer((const void*)k_trace_closest<32, 1, true>, 32);
-  prefer((const void*)k_trace_shadow<16, 0>, 16);
-  prefer((const void*)k_trace_shadow<24, 0>, 24);
-  prefer((const void*)k_trace_shadow<32, 0>, 32);
-  prefer((const void*)k_trace_closest<16, 1, false>, 16);
-  prefer((const void*)k_trace_closest<24, 1, false>, 24);
-  prefer((const void*)k_trace_closest<32, 1, false>, 32);
-  prefer((const void*)k_trace_shadow<16, 1>, 16);
-  prefer((const void*)k_trace_shadow<24, 1>, 24);
-  prefer((const void*)k_trace_shadow<32, 1>, 32);
-  prefer((const void*)k_trace_rays<16>, 16);
-  prefer((const void*)k_trace_rays<24>, 24);
-  prefer((const void*)k_trace_rays<32>, 32);
-  prefer((const void*)k_occluded_rays<16>, 16);
-  prefer((const void*)k_occluded_rays<24>, 24);
-  prefer((const void*)k_occluded_rays<32>, 32);
+  auto allow = [most](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most); };
+  allow(k_trace_closest<16, 0, false>);
+  allow(k_trace_closest<24, 0, false>);
+  allow(k_trace_closest<32, 0, false>);
+  allow(k_trace_closest<16, 1, true>);
+  allow(k_trace_closest<24, 1, true>);
+  allow(k_trace_closest<32, 1, true>);
+  allow(k_trace_shadow<16, 0>);
+  allow(k_trace_shadow<24, 0>);
+  allow(k_trace_shadow<32, 0>);
+  allow(k_trace_closest<16, 1, false>);
+  allow(k_trace_closest<24, 1, false>);
+  allow(k_trace_closest<32, 1, false>);
+  allow(k_trace_shadow<16, 1>);
+  allow(k_trace_shadow<24, 1>);
+  allow(k_trace_shadow<32, 1>);
+  allow(k_trace_rays<16>);
+  allow(k_trace_rays<24>);
+  allow(k_trace_rays<32>);
+  allow(k_occluded_rays<16>);
+  allow(k_occluded_rays<24>);
+  allow(k_occluded_rays<32>);
 }
 
 }  // namespace olc
