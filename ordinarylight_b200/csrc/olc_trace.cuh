@@ -367,7 +367,10 @@ struct Traversal {
       // one, or none of them has anything else to do.
       const uint32_t group = __activemask();
       const uint32_t leaves = __ballot_sync(group, node < 0);
-      if (node < 0 && leaves != group && __popc(leaves) < OLC_LEAF_LANES) continue;
+      if (node < 0 && leaves != group && __popc(leaves) < OLC_LEAF_LANES) {
+        ++budget;   // waiting is no step of the ray; some other lane of the group takes one
+        continue;
+      }
       int next = OLC_MARKER;   // nothing to enter: take the next node from the stack
       if (node >= 0) {
         // BVH4 node: test the four child boxes, descend into the nearest
