@@ -46,15 +46,16 @@
 #define OLC_NO_INSTANCE 0xffffffffu
 #define OLC_MARKER 0x7fffffff
 #define OLC_TRAVERSAL_BUDGET (1u << 22)
-// Lanes that hold a leaf before a warp tests leaves.  One step in five is a
-// leaf, so with some sixteen lanes walking nearly every step also ran the leaf
-// code, for three of them.  A waiting lane loses a step or two but keeps its
-// order, so nothing is tested that was not before.  0 -> 6 lanes: 1080p
-// instanced frame 6.53 -> 6.48 ms, terrain 11.39 -> 11.19 ms, textured 2.40 ->
-// 2.38 ms, one-sample viewport 0.853 -> 0.865 ms; 4, 8 and 12 lanes: 6.50,
-// 6.50 and 6.55 ms, terrain 11.25, 11.19 and 11.22 ms.  (Stepping the whole warp
-// together, with rays replaced as soon as 8 to 20 lanes idle, was 2-5 %
-// slower: lanes that part hide each other's loads.)
+// Lanes that hold a leaf before a warp tests leaves, in queues long enough for
+// it (kLeafWaitRays).  Lanes part, so a step has 7 to 9 of 32 active, and a
+// leaf's code (a triangle test, or an instance's matrix and ray setup) ran for
+// one or two of them at a time.  A waiting lane loses a step or two but keeps
+// its order, so nothing is tested that was not before, and the wait is no step
+// of its budget.  0 -> 6 lanes: 1080p instanced frame 6.22 -> 6.17 ms, terrain
+// 10.61 -> 10.34 ms, textured 2.22 -> 2.20 ms; 4, 8 and 12 lanes: 6.50, 6.50
+// and 6.55 ms where 6 gave 6.48, terrain 11.25, 11.19 and 11.22 where 6 gave
+// 11.19.  (Stepping the whole warp together, with rays replaced as soon as 8
+// to 20 lanes idle, was 2-5 % slower: lanes that part hide each other's loads.)
 #define OLC_LEAF_LANES 6
 
 struct TraceRay {
@@ -355,6 +356,7 @@ struct Traversal {
     return false;
   }
 
+  template <bool WAIT>
   OLC_D bool advance(const SceneView& s, int iterations, uint32_t& err) {
     // The budget is charged per call, not per iteration (a call may charge
     // more than it uses; the bound only has to end a corrupt walk).
@@ -363,13 +365,15 @@ struct Traversal {
     for (uint32_t it = 0; it < steps; ++it) {
       // `node` is never the instance marker here: a marker is only popped,
       // and the pop below steps past it.
-      // Leaves wait until OLC_LEAF_LANES lanes of those walking together hold
-      // one, or none of them has anything else to do.
-      const uint32_t group = __activemask();
-      const uint32_t leaves = __ballot_sync(group, node < 0);
-      if (node < 0 && leaves != group && __popc(leaves) < OLC_LEAF_LANES) {
-        ++budget;   // waiting is no step of the ray; some other lane of the group takes one
-        continue;
+      if (WAIT) {
+        // leaves wait until OLC_LEAF_LANES lanes of those walking together
+        // hold one, or none of them has anything else to do
+        const uint32_t group = __activemask();
+        const uint32_t leaves = __ballot_sync(group, node < 0);
+        if (node < 0 && leaves != group && __popc(leaves) < OLC_LEAF_LANES) {
+          ++budget;   // waiting is no step of the ray; some other lane of the group takes one
+          continue;
+        }
       }
       int next = OLC_MARKER;   // nothing to enter: take the next node from the stack
       if (node >= 0) {

@@ -145,8 +145,8 @@ struct TraceSchedule<1> {
   static constexpr uint32_t kRefillLanes = 32;
 };
 
-template <int STACK, bool ANY_HIT, int SCHED, class Load, class Store>
-OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, int* smem, Load load, Store store,
+template <int STACK, bool ANY_HIT, int SCHED, bool WAIT, class Load, class Store>
+OLC_D void persistent_trace_loop(const SceneView& s, uint32_t n, uint32_t* cursor, int* smem, Load load, Store store,
                             uint32_t& err) {
   constexpr int kTraceSteps = TraceSchedule<SCHED>::kSteps;
   constexpr uint32_t kRefillLanes = TraceSchedule<SCHED>::kRefillLanes;
@@ -189,11 +189,30 @@ OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, in
       }
     }
     if (__ballot_sync(0xffffffffu, my != 0xffffffffu) == 0u) break;
-    if (my != 0xffffffffu && tr.advance(s, kTraceSteps, err)) {
+    if (my != 0xffffffffu && tr.template advance<WAIT>(s, kTraceSteps, err)) {
       store(my, tr);
       my = 0xffffffffu;
     }
   }
+}
+
+// Queues of fewer rays per warp of the grid than this (two a lane) are traced
+// without the wait for leaf lanes: their launch ends with its longest rays,
+// which a wait lengthens, while in a longer queue the issue slots that it saves
+// serve other rays.  Microseconds a frame, with the wait / without: 600,000
+// paths 832 / 817, 380,000 (terrain of 300 x 300) 788 / 773, 160,000 542 / 528;
+// 920,000 paths 1359 / 1374, 1.04 million 2196 / 2216, 2.3 million (terrain of
+// 1,201 x 1,201) 3431 / 3480, 7.4 million 10,320 / 10,610.  With lines of 48, 64
+// and 96 rays: 823 / 821 / 818, 1362 / 1363 / 1370, 3434 / 3432 / 3435.
+constexpr uint32_t kLeafWaitRays = 64;
+
+template <int STACK, bool ANY_HIT, int SCHED, class Load, class Store>
+OLC_D void persistent_trace(const SceneView& s, uint32_t n, uint32_t* cursor, int* smem, Load load, Store store,
+                            uint32_t& err) {
+  if (n / kLeafWaitRays >= gridDim.x * (blockDim.x >> 5))
+    persistent_trace_loop<STACK, ANY_HIT, SCHED, true>(s, n, cursor, smem, load, store, err);
+  else
+    persistent_trace_loop<STACK, ANY_HIT, SCHED, false>(s, n, cursor, smem, load, store, err);
 }
 
 // Register cap of the traversal kernels: 64 registers hold the traversal
