@@ -97,9 +97,15 @@ OLC_D void setup_ray(TraceRay& r, float3 o, float3 d) {
   if (dkz < 0.0f) { int t = kx; kx = ky; ky = t; }
   r.kp = kx | (ky << 2) | (kz << 4);
   r.o = permuted(o, r.kp);
-  r.sz = fabsf(dkz) < 1e-20f ? 1.0f / dkz : get(r.inv, kz);
+  r.sz = get(r.inv, kz);
   r.sx = quotient(get(d, kx), dkz, r.sz);
   r.sy = quotient(get(d, ky), dkz, r.sz);
+  // an infinite or tiny direction, whose reciprocal or residual is out of range
+  if (!(fabsf(dkz) > 1e-18f && fabsf(dkz) < 1e18f)) {
+    r.sz = 1.0f / dkz;
+    r.sx = get(d, kx) / dkz;
+    r.sy = get(d, ky) / dkz;
+  }
 }
 
 // Watertight ray/triangle test on the slot's float4 triple `tv` (one float4
