@@ -606,8 +606,8 @@ typedef struct olc_bvh_info {
 } olc_bvh_info;
 OLC_API int olc_bvh_info_get(const olc_context* ctx, olc_bvh_info* info);
 
-/* Verify the resident BVH: every triangle reachable once and every child box
- * inside its parent.  bad (host) receives the number of violations. */
+/* Verify the resident BVH: every triangle reachable once, by the binary nodes
+ * and by the nodes that traversal reads, and every child box inside its parent.  bad (host) receives the number of violations. */
 OLC_API int olc_bvh_validate(olc_context* ctx, uint64_t* bad);
 
 #ifdef __cplusplus

@@ -1219,8 +1219,9 @@ void build_bvh4(const BvhNode* nodes, BvhNode4* wide, uint32_t begin, uint32_t c
 namespace {
 // Walk each built BLAS from its root; count how often each slot is reached,
 // leaves outside the BLAS's own slot range, child boxes that do not lie
-// inside the box stored for them in the parent, and BVH4 nodes that differ
-// from the collapse of their BVH2 node.
+// inside the box stored for them in the parent, pairs that are not two
+// neighbouring one-triangle leaves, and BVH4 nodes that differ from the
+// collapse of their BVH2 node.
 __global__ void k_validate(SceneView s, const BlasRange* ranges, uint32_t count, uint32_t* slot_hits,
                            unsigned long long* bad) {
   uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1248,6 +1249,13 @@ __global__ void k_validate(SceneView s, const BlasRange* ranges, uint32_t count,
     }
     BvhNode nd = s.nodes[node];
     int ch[2] = {nd.d.x, nd.d.y};
+    if ((uint32_t)nd.d.z & OLC_COLLAPSE_PAIR) {
+      bool neighbours = true;
+      for (int c = 0; c < 2; ++c)
+        neighbours = neighbours && ch[c] < 0 && ch[c] != OLC_EMPTY_CHILD && olc_leaf_count(ch[c]) == 1u;
+      const int gap = (int)olc_leaf_first(ch[0]) - (int)olc_leaf_first(ch[1]);
+      if (!neighbours || (gap != 1 && gap != -1)) atomicAdd(bad, 1ull);
+    }
     for (int c = 0; c < 2; ++c) {
       if (ch[c] == OLC_EMPTY_CHILD) continue;
       if (ch[c] >= 0) {
@@ -1274,29 +1282,69 @@ __global__ void k_validate(SceneView s, const BlasRange* ranges, uint32_t count,
     }
   }
 }
+
+// The same walk over the BVH4 nodes that traversal reads: count how often each
+// slot is reached through them.
+__global__ void k_validate_wide(SceneView s, const BlasRange* ranges, uint32_t count, uint32_t* slot_hits,
+                                unsigned long long* bad) {
+  uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= count) return;
+  const BlasRange r = ranges[b];
+  int stack[256];
+  int sp = 0;
+  stack[sp++] = (int)r.root;
+  for (uint32_t guard = 0; sp > 0; ++guard) {
+    if (guard > (1u << 26)) {
+      atomicAdd(bad, 1ull);
+      break;
+    }
+    const int4 child = s.wide[stack[--sp]].child;
+    for (int ref : {child.x, child.y, child.z, child.w}) {
+      if (ref == OLC_EMPTY_CHILD) continue;
+      if (ref >= 0) {
+        // a pair has no BVH4 node of its own
+        if (sp < 256 && !((uint32_t)s.nodes[ref].d.z & OLC_COLLAPSE_PAIR)) stack[sp++] = ref;
+        else atomicAdd(bad, 1ull);
+        continue;
+      }
+      const uint32_t first = olc_leaf_first(ref), n = olc_leaf_count(ref);
+      for (uint32_t k = 0; k < n; ++k) {
+        if (first + k < r.slot_begin || first + k >= r.slot_end) atomicAdd(bad, 1ull);
+        else atomicAdd(&slot_hits[first + k], 1u);
+      }
+    }
+  }
+}
 }  // namespace
 
 uint64_t validate_bvh(const SceneView& s, const std::vector<BlasRange>& blas, cudaStream_t stream) {
   uint32_t slots = 0;
   for (const BlasRange& r : blas) slots = std::max(slots, r.slot_end);
-  DeviceBuffer hits(std::max<size_t>(slots, 1) * 4), bad(8), ranges(std::max<size_t>(blas.size(), 1) * sizeof(BlasRange));
-  OLC_CUDA(cudaMemsetAsync(hits.get(), 0, std::max<size_t>(slots, 1) * 4, stream));
+  // slot hits through the BVH2 nodes, then through the BVH4 nodes
+  const size_t words = 2 * std::max<size_t>(slots, 1);
+  DeviceBuffer hits(words * 4), bad(8), ranges(std::max<size_t>(blas.size(), 1) * sizeof(BlasRange));
+  OLC_CUDA(cudaMemsetAsync(hits.get(), 0, words * 4, stream));
   OLC_CUDA(cudaMemsetAsync(bad.get(), 0, 8, stream));
   if (!blas.empty()) {
     OLC_CUDA(cudaMemcpyAsync(ranges.get(), blas.data(), blas.size() * sizeof(BlasRange), cudaMemcpyHostToDevice,
                              stream));
-    k_validate<<<blocks_for(blas.size(), 64), 64, 0, stream>>>(s, ranges.as<BlasRange>(), (uint32_t)blas.size(),
-                                                               hits.as<uint32_t>(), bad.as<unsigned long long>());
+    const uint32_t count = (uint32_t)blas.size();
+    k_validate<<<blocks_for(count, 64), 64, 0, stream>>>(s, ranges.as<BlasRange>(), count, hits.as<uint32_t>(),
+                                                         bad.as<unsigned long long>());
     OLC_LAUNCH_CHECK("k_validate");
+    k_validate_wide<<<blocks_for(count, 64), 64, 0, stream>>>(s, ranges.as<BlasRange>(), count,
+                                                              hits.as<uint32_t>() + words / 2,
+                                                              bad.as<unsigned long long>());
+    OLC_LAUNCH_CHECK("k_validate_wide");
   }
-  std::vector<uint32_t> h(std::max<size_t>(slots, 1));
+  std::vector<uint32_t> h(words);
   unsigned long long nbad = 0;
-  OLC_CUDA(cudaMemcpyAsync(h.data(), hits.get(), h.size() * 4, cudaMemcpyDeviceToHost, stream));
+  OLC_CUDA(cudaMemcpyAsync(h.data(), hits.get(), words * 4, cudaMemcpyDeviceToHost, stream));
   OLC_CUDA(cudaMemcpyAsync(&nbad, bad.get(), 8, cudaMemcpyDeviceToHost, stream));
   OLC_CUDA(cudaStreamSynchronize(stream));
   for (const BlasRange& r : blas)
     for (uint32_t i = r.slot_begin; i < r.slot_end; ++i)
-      if (h[i] != 1u) ++nbad;
+      if (h[i] != 1u || h[words / 2 + i] != 1u) ++nbad;
   return nbad;
 }
 

@@ -150,7 +150,9 @@ struct BlasRange {
 };
 
 // Count structural violations of the resident BVH: every slot of every built
-// BLAS reached exactly once from its root, child boxes inside parent boxes.
+// BLAS reached exactly once from its root, through the BVH2 nodes and through
+// the BVH4 nodes; child boxes inside parent boxes; BVH4 nodes current; pairs
+// neighbours.
 uint64_t validate_bvh(const SceneView& s, const std::vector<BlasRange>& blas, cudaStream_t stream);
 
 }  // namespace olc
