@@ -116,8 +116,10 @@ def test_waiting_for_other_rays_spends_no_step_budget(native_library, cuda_devic
 @pytest.mark.parametrize("extent", [(100.0, 1.0, 100.0), (0.0, 5.0, 1000.0), (1e-3, 1.0, 1e3), (0.0, 0.0, 0.0)])
 def test_morton_cells_of_any_extent_build_a_valid_tree(native_library, cuda_device, extent):
     """Meshes above the host builder's limit whose extents differ by up to
-    10^6, or vanish: the tree validates and rays towards triangle centroids
-    report hits no farther than those triangles (brute force over the aimed one)."""
+    10^6, or vanish: the tree validates and rays that start beside their
+    targets report the oracle's hits."""
+    from oracle import production
+
     count = 140_000
     rng = np.random.default_rng(3)
     centre = rng.uniform(-0.5, 0.5, (count, 1, 3)) * np.asarray(extent)
@@ -126,17 +128,36 @@ def test_morton_cells_of_any_extent_build_a_valid_tree(native_library, cuda_devi
     n = 4000
     aim = rng.integers(0, count, n)
     target = v[aim].astype(np.float64).mean(1)
-    o = target + rng.normal(size=(n, 3)) * (1.0 + np.linalg.norm(extent))
+    o = (target + 3.0 * rng.normal(size=(n, 3))).astype(np.float32)
     d = target - o
     dist = np.linalg.norm(d, axis=1)
+    d = (d / dist[:, None]).astype(np.float32)
     with CudaWavefrontRenderer() as r:
         assert r.validate_bvh(scene) == 0
-        _inst, prim, t, _ = r.trace_closest(scene, o.astype(np.float32), (d / dist[:, None]).astype(np.float32))
+        _inst, prim, t, _ = r.trace_closest(scene, o, d)
+    # a direction rounds by 1e-7 of the few units to a triangle 0.01 wide: all but slivers are hit, none is passed
     hit = prim >= 0
-    # the float32 ray passes a 0.01-sized triangle's centroid within ~1e-7 of its length: all but slivers are hit
-    if np.linalg.norm(extent) < 200:
-        assert hit.mean() > 0.97
-    assert np.all(t[hit] <= dist[hit] * (1 + 1e-4) + 0.05) or np.linalg.norm(extent) >= 200
+    assert hit.mean() > 0.99
+    assert np.all(t[hit] <= dist[hit] * (1 + 1e-6) + 0.02)
+    want, want_t = production.trace(scene, o, d)
+    same = prim == want
+    assert same.mean() > 0.995
+    # another triangle only at the same distance, or where the ray passes an edge of the nearer of the two, each within
+    # four roundings of the coordinates
+    other = np.flatnonzero(~same)
+    slack = 4 * np.spacing(np.abs(o[other]).max(1) + dist[other].astype(np.float32)).astype(np.float64)
+    got_t, exp_t = (np.where(k[other] >= 0, x[other], np.inf).astype(np.float64) for k, x in ((prim, t), (want, want_t)))
+    nearer = v[np.where(got_t < exp_t, prim[other], want[other])].astype(np.float64)
+    for k in range(len(other)):
+        if np.isfinite(got_t[k]) and np.isfinite(exp_t[k]) and abs(got_t[k] - exp_t[k]) <= slack[k]:
+            continue
+        ray = d[other[k]].astype(np.float64)
+        corners = nearer[k] - o[other[k]]
+        edges = np.roll(corners, -1, 0) - corners
+        # distance of the ray's line from each edge's line
+        normal = np.cross(edges, ray)
+        gap = np.abs((corners * normal).sum(1)) / np.linalg.norm(normal, axis=1)
+        assert gap.min() <= slack[k]
 
 
 @pytest.mark.parametrize("n", [32_768, 32_769, 1_048_576, 2_097_153, 34_000_001])

@@ -157,3 +157,81 @@ def test_textured_and_untextured_scenes_mix_in_one_batch(native_library, cuda_de
                 ref = p.render_frame(req.scene, req.camera, req.width, req.height, samples=req.samples,
                                      frame_index=req.frame_index)
             assert img.tobytes() == ref.tobytes()
+
+
+def _textured_room(rng, emission=(0.0, 0.0, 0.0)):
+    """A normal-mapped floor (seen from both sides), textured opaque and glass
+    balls, and one emitter too faint to add to any float32 radiance."""
+    from ordinarylight_b200 import scenes
+
+    n = rng.normal(size=(16, 16, 3)) * np.array([0.3, 0.3, 0.0]) + np.array([0.0, 0.0, 1.0])
+    n /= np.linalg.norm(n, axis=-1, keepdims=True)
+    normal = ol.Texture(np.concatenate([np.round((n * 0.5 + 0.5) * 255.0), np.full((16, 16, 1), 255.0)], -1).astype(np.uint8))
+    maps = dict(base_color_texture=ol.Texture(_texture(rng, 16, 16)), metallic_roughness_texture=ol.Texture(_texture(rng, 8, 8)),
+                occlusion_texture=ol.Texture(_texture(rng, 8, 8)), normal_texture=normal)
+    scene, _ = _textured_floor(dict(base_color=(0.9, 0.8, 0.7), roughness=0.8, metallic=0.5, emission=emission,
+                                    emission_two_sided=True,
+                                    emissive_texture=ol.Texture(_texture(rng, 8, 8)), **maps))
+    v, i, vn = scenes.uv_sphere(32, 17)
+    uv = np.stack([np.arctan2(v[:, 2], v[:, 0]) / np.pi, v[:, 1]], -1).astype(np.float32)
+    ball = scene.create_mesh(v, i, ol.Material(), normals=vn, texcoords=uv)
+    glass = ol.Material(base_color=(0.9, 1.0, 0.95), roughness=0.1, transmission=1.0, ior=1.5,
+                        transmission_texture=ol.Texture(_texture(rng, 8, 8)))
+    scene.add_instances(ball, [ol.Transform.translation((-1.2, 1.3, 0.0)), ol.Transform.translation((1.2, 1.3, 0.5))],
+                        materials=[ol.Material(base_color=(0.8, 0.9, 1.0), roughness=0.6, **maps), glass])
+    scene.add_mesh(np.float32([[-1, 6, -1], [1, 6, -1], [1, 6, 1]]), np.uint32([[0, 1, 2]]),
+                   ol.Material(base_color=(0.0, 0.0, 0.0), emission=(1e-20, 1e-20, 1e-20)))
+    scene.set_environment(ol.EnvironmentLight(color=(0.6, 0.7, 0.9), intensity=1.0))
+    return scene
+
+
+@pytest.mark.parametrize("height", [4.0, -4.0])
+@pytest.mark.parametrize("max_bounces", [1, 4])
+def test_surface_recorded_for_resampling_is_the_one_that_shading_computes(native_library, cuda_device, height,
+                                                                          max_bounces):
+    """With ReSTIR the primary hit's textured surface is looked up once and
+    read back by shading.  Without light sampling, the paths are those of a
+    renderer without ReSTIR, which looks it up in shading: the same images,
+    from above and below the floor, for normal-mapped, occluded, transmissive
+    and (as primary emission, one bounce) emissive surfaces."""
+    rng = np.random.default_rng(17)
+    scene = _textured_room(rng, emission=(2.0, 1.5, 1.0) if max_bounces == 1 else (0.0, 0.0, 0.0))
+    camera = ol.PerspectiveCamera(position=(0.3, height, -7.0), target=(0.0, 0.5, 1.0), vertical_fov_degrees=45.0)
+    images = []
+    for restir in (False, True):
+        with CudaWavefrontRenderer(max_bounces=max_bounces, restir=restir, nee=False) as r:
+            images.append([r.render_frame(scene, camera, 71, 45, samples=2, frame_index=k) for k in range(2)])
+    for plain, resampled in zip(*images):
+        assert np.ptp(plain[..., :3]) > 0.1
+        np.testing.assert_allclose(resampled, plain, rtol=0, atol=1e-12)
+
+
+def test_recorded_surfaces_of_served_chunks_of_growing_size(native_library, cuda_device):
+    """Textured ReSTIR requests beside an untextured one, each larger than the
+    one before, so that the recorded surfaces' memory grows between chunks in
+    flight: the images of plain frames, bit for bit."""
+    from ordinarylight_b200 import scenes
+    from ordinarylight_b200.renderers.cuda import RenderRequest
+
+    scene = _textured_room(np.random.default_rng(18))
+    camera = ol.PerspectiveCamera(position=(0.3, 4.0, -7.0), target=(0.0, 0.5, 1.0), vertical_fov_degrees=45.0)
+    plain_scene, pcam = scenes.instanced_spheres(seed=7, instances=6, segments=24, bands=13, emitters=32, extent=5.0)
+    reqs = [RenderRequest(scene, camera, 24, 16, samples=1, frame_index=1, max_bounces=3),
+            RenderRequest(plain_scene, pcam, 64, 48, samples=2, frame_index=2, max_bounces=3),
+            RenderRequest(scene, camera, 111, 64, samples=2, frame_index=3, max_bounces=3),
+            RenderRequest(scene, camera, 320, 200, samples=3, frame_index=4, max_bounces=3)]
+    with CudaWavefrontRenderer(max_bounces=3, restir=True) as r:
+        images = {}
+        tickets = []
+        for req in reqs:
+            tickets.append(r.submit(req))
+            for ticket, image in r.serve_step():
+                images[ticket] = image
+        while r.queued_tickets():
+            for ticket, image in r.serve_step():
+                images[ticket] = image
+    for req, ticket in zip(reqs, tickets):
+        with CudaWavefrontRenderer(max_bounces=3, restir=True, restir_temporal=False) as p:
+            ref = p.render_frame(req.scene, req.camera, req.width, req.height, samples=req.samples,
+                                 frame_index=req.frame_index)
+        assert images[ticket].tobytes() == ref.tobytes()
