@@ -270,12 +270,14 @@ def emitter_records(scene):
     """Emissive triangles with a power CDF: the records and probabilities of
     Scene.emissive_triangle_data (scene/_core.py:2637-2691), computed with
     array operations.  Returns (records [n, 20] float32, total weight)."""
+    own = getattr(type(scene), "emissive_light_weight", None) is Scene.emissive_light_weight
     lit = [m for m in scene.visible_meshes
-           if np.any(np.asarray(m.material.emission, np.float32) > 0.0) or emission_luminance(m.material) > 0.0]
+           if (np.any(np.asarray(m.material.emission, np.float32) > 0.0) or (own and emission_luminance(m.material) > 0.0))
+           and len(m.indices)]
     parts = [m.world_vertices[m.indices] for m in lit]
     areas = triangle_areas(parts)
     sources = [(m, t, a) for m, t, a in zip(lit, parts, areas)
-               if len(t) and np.any(np.asarray(m.material.emission, np.float32) > 0.0)]
+               if np.any(np.asarray(m.material.emission, np.float32) > 0.0)]
     if not sources:
         return np.zeros((0, 20), np.float32), 0.0
     counts = [len(t) for _m, t, _a in sources]
@@ -301,7 +303,7 @@ def emitter_records(scene):
     rec[:, 16] = cdf.astype(np.float32)
     rec[:, 17] = prob.astype(np.float32)
     rec[:, 18] = np.repeat(np.asarray(sided, np.float32), counts)[keep]
-    if getattr(type(scene), "emissive_light_weight", None) is Scene.emissive_light_weight:
+    if own:
         return rec, emissive_weight(lit, areas)   # the property's own sum, over the areas at hand
     return rec, float(getattr(scene, "emissive_light_weight", total))
 

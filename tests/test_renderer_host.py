@@ -163,3 +163,22 @@ def test_install_cuda_preference_routes_cuda_and_keeps_the_rest(monkeypatch):
 def test_install_cuda_preference_without_the_reference(monkeypatch):
     monkeypatch.setitem(sys.modules, "ordinarylight.renderer._core", None)
     assert install_cuda_preference() is False
+
+
+@pytest.mark.parametrize("indices", [[], np.zeros(0), np.zeros((0, 3), np.uint32)])
+@pytest.mark.parametrize("emission", [(2.0, 2.0, 2.0), 0.0, None])
+def test_emitters_skip_what_emits_nothing(indices, emission):
+    """Scenes are read structurally: a mesh without triangles, however it says
+    so, and a material without emission add no emitter."""
+    from types import SimpleNamespace
+
+    from ordinarylight_b200 import packing
+
+    def mesh(idx, em):
+        return SimpleNamespace(material=SimpleNamespace(emission=em), indices=idx,
+                               world_vertices=np.float32([[0, 0, 0], [1, 0, 0], [0, 1, 0]]))
+
+    lit = mesh(np.uint32([[0, 1, 2]]), (1.0, 1.0, 1.0))
+    alone, weight = packing.emitter_records(SimpleNamespace(visible_meshes=[lit]))
+    records, total = packing.emitter_records(SimpleNamespace(visible_meshes=[lit, mesh(indices, emission)]))
+    assert records.tobytes() == alone.tobytes() and total == weight == 0.5
