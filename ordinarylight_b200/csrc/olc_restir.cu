@@ -585,7 +585,7 @@ void restir_prepare(RestirState& st, uint64_t reservoirs, uint32_t slots, uint32
     st.hit_list.allocate((size_t)slots * 4);
     st.slots = slots;
   }
-  if (textures) st.surfaces.ensure((size_t)st.slots * 64);
+  if (textures) st.surfaces.ensure((size_t)slots * 64);   // this run's paths: an earlier, larger run may have had no textures
   if (!st.hit_count.get()) st.hit_count.allocate(32);
   if ((uint64_t)st.next_stamp + chunks >= 0xffffffffull) {
     // stamps would wrap: clear every stored stamp and start again at 1

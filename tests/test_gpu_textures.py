@@ -235,3 +235,17 @@ def test_recorded_surfaces_of_served_chunks_of_growing_size(native_library, cuda
             ref = p.render_frame(req.scene, req.camera, req.width, req.height, samples=req.samples,
                                  frame_index=req.frame_index)
         assert images[ticket].tobytes() == ref.tobytes()
+
+
+def test_recorded_surfaces_take_memory_for_the_textured_paths_only(native_library, cuda_device):
+    """A small textured ReSTIR frame after a large untextured one records its
+    own paths' surfaces, 64 bytes each, not as many as the large frame's."""
+    from ordinarylight_b200 import scenes
+
+    plain, camera = scenes.instanced_spheres(seed=7, instances=6, segments=24, bands=13, emitters=32, extent=5.0)
+    textured = _textured_room(np.random.default_rng(18))
+    with CudaWavefrontRenderer(max_bounces=2, restir=True) as r:
+        r.render_frame(plain, camera, 640, 480, samples=4)
+        before = r.pool_info()["wavefront_bytes"]
+        r.render_frame(textured, camera, 32, 24, samples=1)
+        assert r.pool_info()["wavefront_bytes"] - before < 64 * 640 * 480 * 4 // 2
