@@ -697,17 +697,18 @@ uint32_t build_hierarchy(uint32_t n, BuildScratch& sc, int is_tlas, const TlasRe
                                                                   sc.sorted_hi.as<float4>());
   OLC_LAUNCH_CHECK("k_gather_sorted_boxes");
   OLC_CUDA(cudaMemsetAsync(sc.flags.get(), 0, sizeof(uint32_t) * (n - 1), stream));
+  float4* plan = sc.centers.as<float4>();   // the centres have become keys; their memory takes the collapse plan
   k_bottom_up<<<blocks_for(n), kThreads, 0, stream>>>((int)n, sc.left.as<int>(), sc.right.as<int>(),
                                                         sc.parent.as<int>(), sc.leaf_parent.as<int>(),
                                                         sc.sorted_lo.as<float4>(), sc.sorted_hi.as<float4>(),
                                                         sc.node_lo.as<float4>(), sc.node_hi.as<float4>(),
-                                                        sc.plan.as<float4>(), is_tlas ? 0 : 1,
+                                                        plan, is_tlas ? 0 : 1,
                                                         sc.flags.as<uint32_t>());
   OLC_LAUNCH_CHECK("k_bottom_up");
   k_emit_nodes<<<blocks_for(n - 1), kThreads, 0, stream>>>(
       (int)n, sc.left.as<int>(), sc.right.as<int>(), sc.first.as<int>(), sc.last.as<int>(),
       sc.sorted_lo.as<float4>(), sc.sorted_hi.as<float4>(), sc.node_lo.as<float4>(), sc.node_hi.as<float4>(),
-      sc.plan.as<float4>(), sc.vals.as<uint32_t>(), is_tlas, tr, leaf_max, nodes, node_base, slot_base);
+      plan, sc.vals.as<uint32_t>(), is_tlas, tr, leaf_max, nodes, node_base, slot_base);
   OLC_LAUNCH_CHECK("k_emit_nodes");
   return node_base;  // Karras root is internal node 0
 }
@@ -737,7 +738,6 @@ void BuildScratch::ensure(size_t n) {
   flags.allocate(c * 4);
   node_lo.allocate(c * 16);
   node_hi.allocate(c * 16);
-  plan.allocate(c * 16);
   capacity = c;
 }
 

@@ -72,13 +72,12 @@ class DeviceBuffer {
 // Scratch for one LBVH build of up to n primitives.
 struct BuildScratch {
   DeviceBuffer boxes_lo, boxes_hi;   // float4 per primitive (unsorted)
-  DeviceBuffer centers;              // float4 per primitive
+  DeviceBuffer centers;              // float4 per primitive; then float4 per internal node: collapse costs and word
   DeviceBuffer bounds;               // 6 ordered uints
   DeviceBuffer keys, vals, keys_alt, vals_alt, hist;
   DeviceBuffer sorted_lo, sorted_hi; // float4 per leaf in sorted order
   DeviceBuffer left, right, first, last, parent, leaf_parent, flags;
   DeviceBuffer node_lo, node_hi;     // float4 per internal node
-  DeviceBuffer plan;                 // float4 per internal node: collapse costs and word
   size_t capacity = 0;
   void ensure(size_t n);
 };
