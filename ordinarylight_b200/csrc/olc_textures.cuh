@@ -41,8 +41,9 @@ OLC_D int wrap_index(int value, int size, uint32_t mode) {
   return value;
 }
 
-// v / 255 for a byte value: a reciprocal product and one correction, equal to
-// the rounded quotient for all 256 values.
+// v / 255 for a byte value: a reciprocal product and one residual correction
+// (Markstein, IBM Journal of Research and Development 34(1), 1990), equal to
+// the rounded quotient for all 256 values (tests/test_gpu_arithmetic.py).
 OLC_D float unorm8(uint32_t v) {
   const float x = (float)v, k = 1.0f / 255.0f;
   const float q = __fmul_rn(x, k);
@@ -191,8 +192,8 @@ struct TexturedHit {
 // a resampling pass does, so the initial pass, which needs them first, leaves
 // what they give for the spatial passes and the bounce-0 shading.  The same
 // values they would compute: the footprint of a camera ray is 0 everywhere.
-// 64 bytes written and read twice against two more rounds of lookups: a
-// 960x540 frame of 2 samples 2.71 -> 2.48 ms.
+// 64 bytes (13 of 16 floats used) written and read twice against two more
+// rounds of lookups: a 960x540 frame of 2 samples 2.71 -> 2.48 ms.
 struct SurfaceRecord {
   float3 base, emission, n;   // n: shading normal on the viewer's side
   float roughness, metallic, transmission, occlusion;

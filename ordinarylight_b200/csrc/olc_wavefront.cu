@@ -405,9 +405,9 @@ OLC_D bool next_event(const SceneView& s, const SceneRec& sc, const SurfaceMat& 
 // threads per SM) with media, 72 (seven) without.  kTextures: a variant for
 // runs with a textured scene; the untextured one carries none of the texture
 // code's registers.  kMedia: the same for participating media (delta
-// tracking at the vertex, ratio tracking of the shadow ray), whose code
-// raises the uncapped kernel from 90 to 110 registers (312 bytes of spills
-// at 80 registers with it, 96 at 72 without it).
+// tracking at the vertex, ratio tracking of the shadow ray).  Bytes of spill
+// stores: 132 at 72 registers without media and textures, 268 with textures;
+// 424 at 80 registers with media, 420 with both.
 template <bool kMedia>
 struct ShadeRegisters {
   static constexpr int kCap = kMedia ? 80 : 72;
