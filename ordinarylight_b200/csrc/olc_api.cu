@@ -318,6 +318,7 @@ struct olc_context {
   DeviceBuffer q0_o, q0_d, q0_p, q1_o, q1_d, q1_p, q2_o, q2_d, q2_p, hit_tuv, hit_inst, sh_o, sh_d, sh_c, sh1_o,
       sh1_d, sh1_c, ps_tp, ps_rad, ps_shadow, ps_meta, ps_ior, ps_cone, sort_keys, sort_bins;
   DeviceBuffer counters, job_dev;
+  uint32_t* query_error = nullptr;   // page-locked: set by a ray query's kernel, so that no copy has to fetch it
   DeviceBuffer prod_depth, prod_normal, prod_inst, prod_mat, prod_prim, prod_pos, prod_bary, prod_signals,
       prod_secondary;
   uint32_t prod_pixels = 0;
@@ -1834,14 +1835,19 @@ bool same_camera(const JobRec& a, const JobRec& b) {
          same(a.cam_up, b.cam_up) && a.projection == b.projection;
 }
 
+// Clear what a ray query counts.
+void begin_query(olc_context* ctx) {
+  if (!ctx->counters.get()) ctx->counters.allocate(sizeof(Counters));
+  if (!ctx->query_error) OLC_CUDA(cudaMallocHost(&ctx->query_error, sizeof(uint32_t)));
+  *ctx->query_error = 0u;   // (every query waits for its kernel: none is in flight)
+  OLC_CUDA(cudaMemsetAsync(ctx->counters.get(), 0, sizeof(Counters), ctx->stream));
+}
+
 // Wait for the ray query in flight; a ray whose stack overflowed or whose step
 // budget ran out has no answer.
 void finish_query(olc_context* ctx) {
-  uint32_t errors = 0;
-  OLC_CUDA(cudaMemcpyAsync(&errors, &ctx->counters.as<Counters>()->traversal_errors, sizeof(errors),
-                           cudaMemcpyDeviceToHost, ctx->stream));
   OLC_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (errors) throw Error(OLC_ERR_RUNTIME, "traversal stack overflow");
+  if (*ctx->query_error) throw Error(OLC_ERR_RUNTIME, "traversal stack overflow");
 }
 
 }  // namespace
@@ -1917,6 +1923,7 @@ int olc_destroy(olc_context* ctx) {
   drop_graphs(ctx);
   restir_release(ctx->restir);
   for (RunSlot& sl : ctx->runs) release_slot(sl);
+  if (ctx->query_error) cudaFreeHost(ctx->query_error);
   if (ctx->side) cudaStreamSynchronize(ctx->side);
   cudaStream_t st = ctx->stream, side = ctx->side;
   cudaEvent_t fork = ctx->fork_event, join0 = ctx->join_event[0], join1 = ctx->join_event[1];
@@ -2477,10 +2484,9 @@ int olc_trace_closest(olc_context* ctx, uint32_t n, const float* origins, const 
     const ResidentScene& rs = default_scene(ctx);
     if (n == 0) return;
     if (!origins || !directions) throw Error(OLC_ERR_VALUE, "origins and directions are required");
-    if (!ctx->counters.get()) ctx->counters.allocate(sizeof(Counters));
-    OLC_CUDA(cudaMemsetAsync(ctx->counters.get(), 0, sizeof(Counters), ctx->stream));
+    begin_query(ctx);
     launch_trace_rays(ctx->ls, pool_view(ctx), rs.rec.tlas_root, n, origins, directions, t_min, instance_id,
-                      primitive, t, barycentrics, ctx->counters.as<Counters>(), ctx->stream);
+                      primitive, t, barycentrics, ctx->counters.as<Counters>(), ctx->query_error, ctx->stream);
     finish_query(ctx);
   });
 }
@@ -2492,10 +2498,9 @@ int olc_trace_occluded(olc_context* ctx, uint32_t n, const float* origins, const
     const ResidentScene& rs = default_scene(ctx);
     if (n == 0) return;
     if (!origins || !directions || !t_max || !occluded) throw Error(OLC_ERR_VALUE, "all arrays are required");
-    if (!ctx->counters.get()) ctx->counters.allocate(sizeof(Counters));
-    OLC_CUDA(cudaMemsetAsync(ctx->counters.get(), 0, sizeof(Counters), ctx->stream));
+    begin_query(ctx);
     launch_occluded_rays(ctx->ls, pool_view(ctx), rs.rec.tlas_root, n, origins, directions, t_min, t_max, occluded,
-                         ctx->counters.as<Counters>(), ctx->stream);
+                         ctx->counters.as<Counters>(), ctx->query_error, ctx->stream);
     finish_query(ctx);
   });
 }

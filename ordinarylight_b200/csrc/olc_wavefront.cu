@@ -1067,13 +1067,13 @@ __global__ void k_camera_rays(const JobRec* __restrict__ job_ptr, uint32_t sampl
 }
 
 // Closest hits of caller-supplied rays, with the wavefront's persistent
-// traversal.
+// traversal.  *error is set where some ray was not finished.
 template <int STACK>
 __global__ void __maxnreg__(kTraceRegisters) k_trace_rays(SceneView s, uint32_t root_node, uint32_t n,
                                                           const float* __restrict__ origins,
                                                           const float* __restrict__ dirs, float t_min,
                                                           uint32_t* inst_id, int32_t* prim, float* tout, float* bary,
-                                                          Counters* cnt) {
+                                                          Counters* cnt, uint32_t* error) {
   extern __shared__ int smem_stack[];
   uint32_t err = 0;
   persistent_trace<STACK, false, 0>(
@@ -1098,7 +1098,7 @@ __global__ void __maxnreg__(kTraceRegisters) k_trace_rays(SceneView s, uint32_t 
         }
       },
       err);
-  if (err) atomicAdd(&cnt->traversal_errors, 1u);
+  if (err) *error = 1u;
 }
 
 template <int STACK>
@@ -1106,7 +1106,7 @@ __global__ void __maxnreg__(kTraceRegisters) k_occluded_rays(SceneView s, uint32
                                                              const float* __restrict__ origins,
                                                              const float* __restrict__ dirs, float t_min,
                                                              const float* __restrict__ t_max, uint8_t* occ,
-                                                             Counters* cnt) {
+                                                             Counters* cnt, uint32_t* error) {
   extern __shared__ int smem_stack[];
   uint32_t err = 0;
   persistent_trace<STACK, true, 0>(
@@ -1119,7 +1119,7 @@ __global__ void __maxnreg__(kTraceRegisters) k_occluded_rays(SceneView s, uint32
         root = root_node;
       },
       [&](uint32_t i, const Traversal<STACK, true>& tr) { occ[i] = tr.found() ? 1 : 0; }, err);
-  if (err) atomicAdd(&cnt->traversal_errors, 1u);
+  if (err) *error = 1u;
 }
 
 constexpr int kTraceThreads = 128;
@@ -1309,24 +1309,24 @@ void launch_camera_rays(const LaunchShape& ls, const JobRec* job, uint32_t sampl
 
 void launch_trace_rays(const LaunchShape& ls, const SceneView& s, uint32_t root, uint32_t n, const float* origins,
                        const float* dirs, float t_min, uint32_t* inst_id, int32_t* prim, float* t, float* bary,
-                       Counters* cnt, cudaStream_t stream) {
+                       Counters* cnt, uint32_t* error, cudaStream_t stream) {
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
     const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
     launch_traversal(k_trace_rays<D>, grid, kTraceThreads, D, stream, s, root, n, origins, dirs, t_min, inst_id, prim, t,
-                     bary, cnt);
+                     bary, cnt, error);
   });
   OLC_LAUNCH_CHECK("k_trace_rays");
 }
 
 void launch_occluded_rays(const LaunchShape& ls, const SceneView& s, uint32_t root, uint32_t n, const float* origins,
                           const float* dirs, float t_min, const float* t_max, uint8_t* occ, Counters* cnt,
-                          cudaStream_t stream) {
+                          uint32_t* error, cudaStream_t stream) {
   dispatch_stack(ls.stack_depth, [&](auto depth) {
     constexpr int D = decltype(depth)::value;
     const uint32_t grid = std::min<uint32_t>(n, ls.grid_trace);   // few rays: one per warp
     launch_traversal(k_occluded_rays<D>, grid, kTraceThreads, D, stream, s, root, n, origins, dirs, t_min, t_max, occ,
-                     cnt);
+                     cnt, error);
   });
   OLC_LAUNCH_CHECK("k_occluded_rays");
 }

@@ -127,11 +127,12 @@ void launch_sample_textures(const LaunchShape& ls, const SceneRec* scenes, uint3
                             float4* out, cudaStream_t stream);
 void launch_camera_rays(const LaunchShape& ls, const JobRec* job, uint32_t sample, const float* jitter,
                         float* origins, float* dirs, cudaStream_t stream);
+// *error (page-locked host memory, cleared by the caller) is set where some ray was not finished.
 void launch_trace_rays(const LaunchShape& ls, const SceneView& s, uint32_t root, uint32_t n, const float* origins,
                        const float* dirs, float t_min, uint32_t* inst_id, int32_t* prim, float* t, float* bary,
-                       Counters* cnt, cudaStream_t stream);
+                       Counters* cnt, uint32_t* error, cudaStream_t stream);
 void launch_occluded_rays(const LaunchShape& ls, const SceneView& s, uint32_t root, uint32_t n, const float* origins,
                           const float* dirs, float t_min, const float* t_max, uint8_t* occ, Counters* cnt,
-                          cudaStream_t stream);
+                          uint32_t* error, cudaStream_t stream);
 
 }  // namespace olc
