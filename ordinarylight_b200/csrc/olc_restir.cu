@@ -396,7 +396,7 @@ __global__ void k_restir_pool(const ChunkHeader* __restrict__ hdr, const JobRec*
 }
 
 // Eight blocks of 128 threads per SM for the untextured kernel (64
-// registers, 20 bytes of spills outside the candidate loop): the candidate
+// registers, no spills): the candidate
 // loop is issue-bound and gains from the extra warps (1.657 -> 1.625 ms of
 // ReSTIR per 1080p frame).  The textured kernel keeps its 128 registers.
 template <bool kTextures>
@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(128, kTextures ? 4 : 8) k_restir_initial(Resti
   }
 }
 
-// Eight blocks of 128 threads per SM for the untextured kernel too (64
-// registers instead of 69, 20 bytes of spills): with its grid one resident
+// Eight blocks of 128 threads per SM (64 registers instead of 69, 16 bytes
+// of spills): with its grid one resident
 // wave, the eighth block per SM took its ReSTIR time from 1.495 to 1.468 ms
 // per 1080p instanced frame.
 template <bool kTextures>
